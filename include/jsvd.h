@@ -132,7 +132,7 @@ int jsvd_auto_tune_layout(const jsvd_config *cfg, jsvd_autotune_report *report);
 typedef struct jsvd_plain_stats {
     unsigned long long solves;
     unsigned long long sweeps;
-    unsigned long long round_launches;
+    unsigned long long round_launches; /* several rounds each up to 1024 rows */
     unsigned long long vpass_launches;
     unsigned long long other_launches; /* layout, identity, sigma, U and V kernels */
     double round_ms;

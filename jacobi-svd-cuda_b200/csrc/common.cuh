@@ -92,6 +92,21 @@ __host__ __device__ __forceinline__ int circle_col(int n, int L, int r, int pos)
     return c == n ? -1 : c;
 }
 
+// circle_col for 0 <= r < L and 0 <= pos < ne, without a division.
+__host__ __device__ __forceinline__ int circle_col_near(int n, int L, int r, int pos)
+{
+    if (pos == 0) return 0;
+    const int v = pos - 1 - r;
+    const int c = 1 + (v < 0 ? v + L : v);
+    return c == n ? -1 : c;
+}
+
+// Barrier `id` (1..15) among `threads` threads of the block.
+__device__ __forceinline__ void group_barrier(int id, int threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // Rutishauser rotation for the 2x2 Gram [pp pq; pq qq]; returns true when the
 // pair rotates.  A pair that does not rotate reports c = 0, s = 0 (a real
 // rotation always has c >= 1/sqrt(2)), which is how the deferred V update
@@ -99,19 +114,21 @@ __host__ __device__ __forceinline__ int circle_col(int n, int L, int r, int pos)
 __device__ __forceinline__ bool rotation_params(double pp, double qq, double pq, double eps, double &c,
                                                 double &s)
 {
+    // The threshold's square root and the angle's chain of divisions and square
+    // roots do not depend on each other: both run unconditionally, side by
+    // side, and the selection comes last (a pair that does not rotate drops
+    // whatever the chain gave, infinities and NaNs included).
     const double rhs = eps * sqrt(fmax(pp, 0.0) * fmax(qq, 0.0));
-    if (fabs(pq) > rhs && fabs(pq) > 1.0e-300) {
-        const double tau = (qq - pp) / (2.0 * pq);
-        const double h = fma(tau, tau, 1.0);
-        const double t = (tau >= 0.0) ? (1.0 / (tau + sqrt(h))) : (-1.0 / (-tau + sqrt(h)));
-        const double cs = 1.0 / sqrt(fma(t, t, 1.0));
-        c = cs;
-        s = t * cs;
-        return true;
-    }
-    c = 0.0;
-    s = 0.0;
-    return false;
+    const double tau = (qq - pp) / (2.0 * pq);
+    const double h = fma(tau, tau, 1.0);
+    // 1 / (|tau| + sqrt(h)) with tau's sign (division is symmetric in the sign)
+    const double r = 1.0 / (fabs(tau) + sqrt(h));
+    const double t = (tau >= 0.0) ? r : -r;
+    const double cs = 1.0 / sqrt(fma(t, t, 1.0));
+    const bool rot = fabs(pq) > rhs && fabs(pq) > 1.0e-300;
+    c = rot ? cs : 0.0;
+    s = rot ? t * cs : 0.0;
+    return rot;
 }
 
 // Halving tree over W = T/32 per-lane register values followed by the

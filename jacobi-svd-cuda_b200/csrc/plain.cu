@@ -6,10 +6,11 @@
 // execution:
 //   * A lives in a column-major working copy (lda = m), so every pair reads two
 //     contiguous columns with fully coalesced accesses.
-//   * One fused kernel per round: Gram dot products (fma chains over T virtual
+//   * One kernel per round, or per several rounds up to 1024 rows
+//     (plain_fused_kernel): Gram dot products (fma chains over T virtual
 //     lanes + the reference's halving tree, warp shuffles for the in-warp
 //     levels), Rutishauser angle in registers, rotation of the register-held
-//     column tiles written back in place.  The reference needs three launches
+//     column tiles.  The reference needs three launches
 //     and three blocking host transfers per round.
 //   * V never sits on the round-to-round critical path.  Each round records
 //     its (c, s); after a sweep that rotated, one row-parallel pass applies the
@@ -209,6 +210,266 @@ __global__ void __launch_bounds__(T) plain_round_kernel(double *__restrict__ a, 
     }
 }
 
+// ---- several rounds per launch -------------------------------------------------
+// Round r + 1 of slot k (slot k pairs circle positions k and ne-1-k) needs two
+// columns, and round r left them in the neighbouring slots: the top one came
+// from slot k-1 and the bottom one from slot k+1.  So a CTA can run R rounds
+// for its slots on its own when it starts from enough pairs around them: level
+// 0 works pairs of round r0, level i those pairs of round r0+i that can be
+// formed from level i-1, the last level the CTA's own slots, which it writes
+// out.  The neighbouring CTAs work the pairs between as well, and nobody waits
+// for anybody: the columns come from one buffer and go to another (the two
+// alternate between launches).  The rounds of an L2-resident matrix are a chain
+// of latencies (launch, column loads, reduction, angle, stores and their
+// flush), and R rounds share the launch, the loads and the stores.
+//
+// Geometry.  A CTA owns S slots k0, k0+2, ..., all of one parity: what a level
+// needs then has one parity too, S + w pairs at x = k0 - w + 2g (group g =
+// 0 .. S-1+w, w = R-1-i rounds to go), so the work is 1 + (R-1) / (2S) times
+// that of R single rounds.  The row of slots reflects at both ends: x < 0 is
+// slot -x-1, x > h (the last slot) is slot 2h+1-x.  At the next level group g
+// stands at x' between its own x and group g+1's, and takes one column from
+// itself and one from group g+1: itself the top and its neighbour the bottom,
+// the other way round where it is reflected.  Those are the same side of the
+// pair they come from, except that slot 1's top was slot 0's bottom (slot 0's
+// top is the fixed column) and the last slot's bottom was its own top.  So
+// each group publishes one column per level, the one its left neighbour wants.
+//
+// G threads work one pair; thread t holds the reference's virtual lanes
+// t, t + G, ... (T = 256 of them) and K rows of each, in registers from the
+// loads to the stores, so the sums meet in the reference's order: the levels
+// T/2 .. G of the halving tree in registers, G/2 .. 32 through shared memory,
+// 16 .. 1 by shuffles (an xor butterfly: the operands of an addition commute,
+// and every lane ends with the total).  JU of a thread's T/G lanes can hold rows
+// (m <= JU G when K = 1); the others' zeros leave the tree as it is.
+constexpr int kFusedT = 256;
+constexpr int kFusedMaxThreads = 512;
+constexpr size_t kFusedSmemCap = 128 * 1024;  // 6 groups of 1024 rows, two levels: 96 KiB
+
+// Slot of a group at x, and whether it is reflected (half = h + 1 slots).
+__host__ __device__ __forceinline__ int fused_slot(int x, int half, bool &mirrored)
+{
+    mirrored = x < 0 || x >= half;
+    return x < 0 ? -x - 1 : (x >= half ? 2 * half - 1 - x : x);
+}
+
+// Columns in shared memory are padded to the rows a group's registers cover.
+template <int G, int JU, int K>
+constexpr int kFusedRows = G * JU + kFusedT * (K - 1);
+
+template <int G, int JU, int K>
+__global__ void __launch_bounds__(kFusedMaxThreads, 1)
+    plain_fused_kernel(const double *a_in, double *a_out, long lda, int m, int n, int R,
+                       int S, int r0, double2 *__restrict__ cs, int npairs, double eps,
+                       unsigned *__restrict__ counter)
+{
+    constexpr int W = G / 32;  // warps per pair
+    constexpr int P = kFusedRows<G, JU, K>;
+    extern __shared__ double xbuf[];  // published columns: [level parity][group][P]
+    __shared__ double red[W > 1 ? 3 * kFusedMaxThreads : 1];
+    __shared__ double2 cs_sh[W > 2 ? kFusedMaxThreads / G : 1];
+    pdl_launch_dependents();
+    const int g = threadIdx.x / G, t = threadIdx.x % G;
+    const int ne = n + (n & 1), half = ne / 2, L = ne - 1;
+    const int k0 = (blockIdx.x & 1) + 2 * (blockIdx.x >> 1) * S;
+    const int own = min(S, (half - k0 + 1) >> 1);  // slots of this CTA
+    if (own <= 0) return;
+    const int groups = S + R - 1;
+    const int last = k0 + 2 * (own - 1);
+
+    double xp[JU][K], xq[JU][K];  // rows t + G j + T i of the top and the bottom column
+    // Where this group stands at level `lev`.  The next level's is worked out
+    // beside the angle's chain, off the path from barrier to barrier.
+    int x = k0 - (R - 1) + 2 * g;
+    int slot, dummy = n + r0;
+    bool mir, real, writer;
+    double2 *cs_row = cs + (size_t)r0 * npairs, *cs_out;
+    auto stand = [&](int lev) {
+        slot = fused_slot(x, half, mir);
+        // the dummy column's slot (odd n) has no pair
+        const int pos = dummy > L ? dummy - L : dummy;
+        const int dslot = (n & 1) ? (pos < half ? pos : L - pos) : half;
+        real = slot != dslot;
+        cs_out = cs_row + (slot - (slot > dslot ? 1 : 0));
+        // every pair of a round is recorded by one CTA: slot k by its owner
+        // where a group stands at it, else by the owner of slot k - 1 (slot 0
+        // by its own owner's reflected group)
+        writer = real && (((R - 1 - lev) & 1) ? ((x > k0 && x <= last + 1 && x < half) || (k0 == 0 && x == -1))
+                                              : (x >= k0 && x <= last));
+    };
+    stand(0);
+    {
+        const int p = circle_col_near(n, L, r0, slot), q = circle_col_near(n, L, r0, ne - 1 - slot);
+        const double *ap = a_in + (size_t)max(p, 0) * lda;
+        const double *aq = a_in + (size_t)max(q, 0) * lda;
+        const bool live = g < own + R - 1;
+        // The previous launch's columns, through L2: a launch that began before
+        // the previous one ended may share an SM, and its L1, with it.
+        pdl_wait();
+#pragma unroll
+        for (int j = 0; j < JU; ++j)
+#pragma unroll
+            for (int i = 0; i < K; ++i) {
+                const int row = t + G * j + kFusedT * i;
+                xp[j][i] = (live && row < m) ? __ldcg(ap + row) : 0.0;
+                xq[j][i] = (live && row < m) ? __ldcg(aq + row) : 0.0;
+            }
+    }
+    double *pub = xbuf + (size_t)g * P + t;
+    const double *nbr = pub + P;
+    long flip = (long)groups * P;
+    for (int lev = 0;; ++lev) {
+        const int w = R - 1 - lev;
+        if (g < own + w) {
+            // what the left neighbour wants of this pair at the next level
+            bool pmir;
+            const int pslot = fused_slot(x - 1, half, pmir);
+            const bool want_top = pmir ? pslot != 1 : pslot == half - 1;
+            const bool work = real, record = writer && t == 0;
+            double2 *const cs_now = cs_out;
+            const int p = circle_col_near(n, L, r0 + lev, slot), q = circle_col_near(n, L, r0 + lev, ne - 1 - slot);
+            double spp[JU], sqq[JU], spq[JU];
+#pragma unroll
+            for (int j = 0; j < JU; ++j) {
+                spp[j] = sqq[j] = spq[j] = 0.0;
+#pragma unroll
+                for (int i = 0; i < K; ++i) {  // rows past m are zero: they leave the sums as they are
+                    spp[j] = fma(xp[j][i], xp[j][i], spp[j]);
+                    sqq[j] = fma(xq[j][i], xq[j][i], sqq[j]);
+                    spq[j] = fma(xp[j][i], xq[j][i], spq[j]);
+                }
+            }
+#pragma unroll
+            for (int d = JU / 2; d >= 1; d >>= 1)
+#pragma unroll
+                for (int j = 0; j < d; ++j) {
+                    spp[j] += spp[j + d];
+                    sqq[j] += sqq[j + d];
+                    spq[j] += spq[j + d];
+                }
+            double pp = spp[0], qq = sqq[0], pq = spq[0], c, s;
+            auto angle = [&]() {
+#pragma unroll
+                for (int off = 16; off >= 1; off >>= 1) {
+                    pp += __shfl_xor_sync(0xffffffffu, pp, off);
+                    qq += __shfl_xor_sync(0xffffffffu, qq, off);
+                    pq += __shfl_xor_sync(0xffffffffu, pq, off);
+                }
+                rotation_params(pp, qq, pq, eps, c, s);
+            };
+            ++x;
+            ++dummy;
+            cs_row += npairs;
+            stand(lev + 1);
+            if constexpr (W > 1) {
+                double *rg = red + g * 3 * G;
+                rg[t] = pp;
+                rg[G + t] = qq;
+                rg[2 * G + t] = pq;
+                group_barrier(1 + g, G);
+                if (W == 2 || t < 32) {
+                    double y[3][W];
+#pragma unroll
+                    for (int v = 0; v < 3; ++v) {
+#pragma unroll
+                        for (int u = 0; u < W; ++u) y[v][u] = rg[v * G + 32 * u + (t & 31)];
+#pragma unroll
+                        for (int d = W / 2; d >= 1; d >>= 1)
+#pragma unroll
+                            for (int u = 0; u < d; ++u) y[v][u] += y[v][u + d];
+                    }
+                    pp = y[0][0];
+                    qq = y[1][0];
+                    pq = y[2][0];
+                    angle();
+                    if (W > 2 && t == 0) cs_sh[g] = make_double2(c, s);
+                }
+                if constexpr (W > 2) {
+                    group_barrier(1 + g, G);
+                    c = cs_sh[g].x;
+                    s = cs_sh[g].y;
+                }
+            } else {
+                angle();
+            }
+            const bool rot = work && c != 0.0;
+            if (rot) {
+#pragma unroll
+                for (int j = 0; j < JU; ++j)
+#pragma unroll
+                    for (int i = 0; i < K; ++i) {
+                        const double xv = xp[j][i], yv = xq[j][i];
+                        xp[j][i] = rot_p(c, s, xv, yv);
+                        xq[j][i] = rot_q(c, s, xv, yv);
+                    }
+            }
+            if (w > 0) {
+                if (g > 0) {
+                    if (want_top) {
+#pragma unroll
+                        for (int j = 0; j < JU; ++j)
+#pragma unroll
+                            for (int i = 0; i < K; ++i) pub[G * j + kFusedT * i] = xp[j][i];
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < JU; ++j)
+#pragma unroll
+                            for (int i = 0; i < K; ++i) pub[G * j + kFusedT * i] = xq[j][i];
+                    }
+                }
+            } else {
+                double *op = a_out + (size_t)max(p, 0) * lda;
+                double *oq = a_out + (size_t)max(q, 0) * lda;
+#pragma unroll
+                for (int j = 0; j < JU; ++j)
+#pragma unroll
+                    for (int i = 0; i < K; ++i) {
+                        const int row = t + G * j + kFusedT * i;
+                        if (row < m) {
+                            if (p >= 0) op[row] = xp[j][i];
+                            if (q >= 0) oq[row] = xq[j][i];
+                        }
+                    }
+            }
+            if (record) {
+                *cs_now = make_double2(c, s);
+                if (rot) atomicAdd(counter, 1u);
+            }
+        }
+        if (w == 0) break;
+        __syncthreads();
+        if (g < own + w - 1) {
+            // this level's pair from the last one's: see the geometry above
+            if (!mir) {
+                if (slot == 1) {
+#pragma unroll
+                    for (int j = 0; j < JU; ++j)
+#pragma unroll
+                        for (int i = 0; i < K; ++i) xp[j][i] = xq[j][i];
+                }
+#pragma unroll
+                for (int j = 0; j < JU; ++j)
+#pragma unroll
+                    for (int i = 0; i < K; ++i) xq[j][i] = nbr[G * j + kFusedT * i];
+            } else {
+                if (slot == half - 1) {
+#pragma unroll
+                    for (int j = 0; j < JU; ++j)
+#pragma unroll
+                        for (int i = 0; i < K; ++i) xq[j][i] = xp[j][i];
+                }
+#pragma unroll
+                for (int j = 0; j < JU; ++j)
+#pragma unroll
+                    for (int i = 0; i < K; ++i) xp[j][i] = nbr[G * j + kFusedT * i];
+            }
+        }
+        pub += flip;
+        nbr += flip;
+        flip = -flip;
+    }
+}
+
 // Counts the pairs p > q of the lower triangle of G (column-major, ld n) that
 // pass the reference's rotation test (src/kernels.cu:503-505):
 // |g_pq| > eps sqrt(max(g_pp, 0) max(g_qq, 0)) and |g_pq| > 1e-300.
@@ -241,9 +502,9 @@ __global__ void gram_offdiag_count(const double *__restrict__ G, int n, double e
 // round are disjoint and the barrier between rounds makes each round's global
 // stores visible to the block, so the sequence of rotations per element, and
 // so the result, is the same.
-constexpr int kVpassSlots = 8;  // prefetched pair slots per thread and round
+constexpr int kVpassSlots = 8;  // most prefetched pair slots per thread and round
 
-template <int R, bool kStaged>
+template <int R, int Q, bool kStaged>
 __global__ void __launch_bounds__(512) plain_vpass_kernel(double *__restrict__ v, long ldv, int n,
                                                           const double2 *__restrict__ cs, int rounds, int npairs)
 {
@@ -264,32 +525,32 @@ __global__ void __launch_bounds__(512) plain_vpass_kernel(double *__restrict__ v
         __syncthreads();
     }
     // Thread k0 owns pair slots k0, k0 + blockDim.x, ...: the (c, s) of its
-    // first kVpassSlots slots for round r + 1 are loaded while round r is
+    // first Q slots for round r + 1 are loaded while round r is
     // applied, so a round waits on one L2 round trip, not one per slot (the
     // loads cannot move past the shared-memory stores of the previous slot).
-    // Slots beyond those (more than kVpassSlots * blockDim.x pairs) are read
+    // Slots beyond those (more than Q * blockDim.x pairs) are read
     // when used.
     const int k0 = threadIdx.x;
     const int nb = blockDim.x;
-    double2 g_next[kVpassSlots];
+    double2 g_next[Q];
 #pragma unroll
-    for (int j = 0; j < kVpassSlots; ++j) {
+    for (int j = 0; j < Q; ++j) {
         const int k = k0 + j * nb;
         g_next[j] = (k < npairs) ? cs[k] : make_double2(0.0, 0.0);
     }
     for (int r = 0; r < rounds; ++r) {
-        double2 g_cur[kVpassSlots];
+        double2 g_cur[Q];
 #pragma unroll
-        for (int j = 0; j < kVpassSlots; ++j) g_cur[j] = g_next[j];
+        for (int j = 0; j < Q; ++j) g_cur[j] = g_next[j];
         if (r + 1 < rounds) {
 #pragma unroll
-            for (int j = 0; j < kVpassSlots; ++j) {
+            for (int j = 0; j < Q; ++j) {
                 const int k = k0 + j * nb;
                 if (k < npairs) g_next[j] = cs[(size_t)(r + 1) * npairs + k];
             }
         }
 #pragma unroll
-        for (int j = 0; j < kVpassSlots; ++j) {
+        for (int j = 0; j < Q; ++j) {
             const int k = k0 + j * nb;
             const double2 g = g_cur[j];
             if (k < npairs && g.x != 0.0) {
@@ -307,7 +568,7 @@ __global__ void __launch_bounds__(512) plain_vpass_kernel(double *__restrict__ v
                 }
             }
         }
-        for (int k = k0 + kVpassSlots * nb; k < npairs; k += nb) {
+        for (int k = k0 + Q * nb; k < npairs; k += nb) {
             const double2 g = cs[(size_t)r * npairs + k];
             if (g.x != 0.0) {
                 const int2 pq = round_robin_pair(n, r, k);
@@ -542,15 +803,25 @@ using RoundFn = void (*)(double *, long, int, const int2 *, double2 *, double, u
 using SigmaFn = void (*)(const double *, long, int, double *);
 using VpassFn = void (*)(double *, long, int, const double2 *, int, int);
 
-VpassFn pick_vpass(int R, bool staged)
+template <int Q>
+VpassFn pick_vpass_q(int R, bool staged)
 {
-    if (!staged) return plain_vpass_kernel<1, false>;
+    if (!staged) return plain_vpass_kernel<1, Q, false>;
     switch (R) {
-    case 1: return plain_vpass_kernel<1, true>;
-    case 2: return plain_vpass_kernel<2, true>;
-    case 4: return plain_vpass_kernel<4, true>;
-    default: return plain_vpass_kernel<8, true>;
+    case 1: return plain_vpass_kernel<1, Q, true>;
+    case 2: return plain_vpass_kernel<2, Q, true>;
+    case 4: return plain_vpass_kernel<4, Q, true>;
+    default: return plain_vpass_kernel<8, Q, true>;
     }
+}
+
+// `slots`: pair slots per thread.
+VpassFn pick_vpass(int R, bool staged, int slots)
+{
+    if (slots <= 1) return pick_vpass_q<1>(R, staged);
+    if (slots <= 2) return pick_vpass_q<2>(R, staged);
+    if (slots <= 4) return pick_vpass_q<4>(R, staged);
+    return pick_vpass_q<kVpassSlots>(R, staged);
 }
 
 template <int T, bool kOnce>
@@ -582,6 +853,61 @@ RoundFn pick_round_o(int T, int m)
 }
 
 RoundFn pick_round(int T, int m, bool once) { return once ? pick_round_o<true>(T, m) : pick_round_o<false>(T, m); }
+
+using FusedFn = void (*)(const double *, double *, long, int, int, int, int, int, double2 *, int, double, unsigned *);
+
+struct FusedKernel {
+    FusedFn fn = nullptr;
+    int threads = 0;  // per pair
+    int rows = 0;     // rows of a column in shared memory
+};
+
+template <int G, int JU, int K>
+FusedKernel fused_kernel()
+{
+    return {plain_fused_kernel<G, JU, K>, G, kFusedRows<G, JU, K>};
+}
+
+// The fused kernel of an m-row matrix: threads per pair, lanes and rows per
+// thread.  One warp per pair up to 256 rows; above, two warps keep a thread at
+// 16 rows or fewer (one warp per pair at 512 rows: 13.2 ms per 512 x 512 solve
+// against 11.3).
+FusedKernel pick_fused(int m)
+{
+    if (m <= 64) return fused_kernel<32, 2, 1>();
+    if (m <= 128) return fused_kernel<32, 4, 1>();
+    if (m <= 256) return fused_kernel<32, 8, 1>();
+    if (m <= 512) return fused_kernel<64, 4, 2>();
+    if (m <= 1024) return fused_kernel<64, 4, 4>();
+    return {};
+}
+
+// Slots per CTA: as many as it takes for one CTA per SM (more slots repeat
+// less of the neighbours' work, fewer would leave SMs idle).  Rounds per
+// launch: 6 - slots, at least 3 (six at up to 256 rows, where a pair's work
+// is small): about five pairs in flight per CTA at the first level; with more
+// the pairs of a level wait on the FP64 pipe, and the CTA no longer fits an SM
+// beside the V pass of the previous sweep (448 threads at 512 x 512: 15.5 ms
+// against 11.3 with 320).  Above 1024 rows the one-round kernel is as fast
+// (2000 x 600: 27.5 ms, two rounds per launch 31.4).  Per solve, one-round
+// kernel -> this (B200): 64 x 48 1.32 -> 0.77 ms, 256 x 256 8.4 -> 4.6, 512 x 512
+// 19.4 -> 11.3, 1000 x 333 11.2 -> 7.4, 1024 x 1024 60.2 -> 40.7.
+struct FusedShape {
+    int rounds = 0, slots = 0;  // rounds 0: one round per launch
+};
+
+FusedShape fused_shape(int m, int n, int sms)
+{
+    const int half = (n + (n & 1)) / 2;
+    FusedShape f;
+    if (pick_fused(m).fn == nullptr || half < 3) return f;
+    f.slots = (half + sms - 1) / sms;
+    f.rounds = std::min(half - 1, m <= 256 ? 6 : std::max(3, 6 - f.slots));
+    return f;
+}
+
+// Dynamic shared memory of the fused kernel: two levels' published columns.
+size_t fused_smem(int rows, int groups) { return sizeof(double) * 2 * (size_t)groups * (size_t)rows; }
 
 SigmaFn pick_sigma(int T)
 {
@@ -661,7 +987,7 @@ PlainPlan::~PlainPlan()
     for (int p = 0; p < 2; ++p)
         for (cudaEvent_t e : {ev_rounds_done[p], ev_vpass_done[p], ev_v0[p], ev_v1[p]})
             if (e) cudaEventDestroy(e);
-    for (void *p : {(void *)a_w, (void *)v_w, (void *)pairs, (void *)cs, (void *)cs2, (void *)counter, (void *)flags,
+    for (void *p : {(void *)a_w, (void *)a_w2, (void *)v_w, (void *)pairs, (void *)cs, (void *)cs2, (void *)counter, (void *)flags,
                     (void *)d_in, (void *)d_u, (void *)d_sigma, (void *)d_v, (void *)sigma_w, (void *)gram,
                     (void *)gram_count})
         if (p) cudaFreeAsync(p, stream);
@@ -720,8 +1046,9 @@ int PlainPlan::create(int dev, size_t m_, size_t n_, int T_, double eps_, cudaSt
         // fixed cap, never to this plan's size, or a plan created concurrently
         // on another thread could lower it under a larger plan's launch.
         if (plan->vpass_staged)
-            JSVD_CUDA_TRY(cudaFuncSetAttribute(pick_vpass(R, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem_cap));
+            for (int q : {1, 2, 4, kVpassSlots})
+                JSVD_CUDA_TRY(cudaFuncSetAttribute(pick_vpass(R, true, q), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem_cap));
         JSVD_CUDA_TRY(cudaEventCreate(&plan->ev_round_begin));
         JSVD_CUDA_TRY(cudaEventCreate(&plan->ev_round_end));
         // Persistent sweep when the whole grid can be co-resident.
@@ -738,8 +1065,18 @@ int PlainPlan::create(int dev, size_t m_, size_t n_, int T_, double eps_, cudaSt
             JSVD_CUDA_TRY(cudaMallocAsync((void **)&plan->flags, sizeof(int) * (plan->sweep_grid + 1), stream));
             plan->persistent = true;
         }
+        const FusedShape fs = fused_shape((int)m_, (int)n_, sms);
+        if (fs.rounds > 0 && T_ == kFusedT && sweep_mode() == 0 &&
+            pick_fused((int)m_).threads * (fs.slots + fs.rounds - 1) <= kFusedMaxThreads) {
+            plan->fused_rounds = fs.rounds;
+            plan->fused_slots = fs.slots;
+            JSVD_CUDA_TRY(cudaMallocAsync((void **)&plan->a_w2, sizeof(double) * m_ * n_, stream));
+            // the same cap for every plan, like the V pass's above
+            JSVD_CUDA_TRY(cudaFuncSetAttribute(pick_fused((int)m_).fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kFusedSmemCap));
+        }
     }
-    plan->bytes = sizeof(double) * (m_ * n_ + n_ * n_ + n_) +
+    plan->bytes = sizeof(double) * ((plan->a_w2 ? 2 : 1) * m_ * n_ + n_ * n_ + n_) +
                   (sizeof(int2) + 2 * sizeof(double2)) * (size_t)plan->rounds * plan->npairs;
     // The allocations become usable on any stream once this one has drained.
     JSVD_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -755,17 +1092,33 @@ int PlainPlan::enqueue_rounds(cudaStream_t st, int parity)
     RoundFn round_fn = pick_round(T, (int)m, angle_once);
     double2 *tab = parity ? cs2 : cs;
     JSVD_CUDA_TRY(cudaEventRecordWithFlags(ev_round_begin, st, sweep_exec_capturing ? cudaEventRecordExternal : 0));
-    // With use_pdl, rounds after the first are launched with programmatic
-    // stream serialisation, so each round's launch overlaps the previous
-    // round's tail.
+    // Programmatic stream serialisation: a launch begins while the previous one
+    // ends, and waits for it before it reads a column.
     cudaLaunchAttribute pdl[1];
     pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     pdl[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t lc = {};
+    lc.stream = st;
+    if (fused_rounds > 0) {
+        const FusedKernel fk = pick_fused((int)m);
+        const int half = (int)((n + (n & 1)) / 2);
+        lc.gridDim = dim3(2 * (((half + 1) / 2 + fused_slots - 1) / fused_slots));
+        int buf = (fused_launches() & 1) ? parity : 0;  // the copy that holds A
+        for (int r = 0; r < rounds; r += fused_rounds, buf ^= 1) {
+            const int R = std::min(fused_rounds, rounds - r), groups = fused_slots + R - 1;
+            lc.blockDim = dim3(fk.threads * groups);
+            lc.dynamicSmemBytes = fused_smem(fk.rows, groups);
+            lc.attrs = r > 0 ? pdl : nullptr;
+            lc.numAttrs = r > 0 ? 1 : 0;
+            JSVD_CUDA_TRY(cudaLaunchKernelEx(&lc, fk.fn, (const double *)(buf ? a_w2 : a_w), buf ? a_w : a_w2, lda,
+                                             (int)m, (int)n, R, fused_slots, r, tab, npairs, eps, counter));
+        }
+        JSVD_CUDA_TRY(
+            cudaEventRecordWithFlags(ev_round_end, st, sweep_exec_capturing ? cudaEventRecordExternal : 0));
+        return JSVD_OK;
+    }
     lc.gridDim = dim3(npairs);
     lc.blockDim = dim3(T);
-    lc.dynamicSmemBytes = 0;
-    lc.stream = st;
     for (int r = 0; r < rounds; ++r) {
         const size_t off = (size_t)r * npairs;
         lc.attrs = r > 0 && use_pdl ? pdl : nullptr;
@@ -781,8 +1134,9 @@ int PlainPlan::enqueue_rounds(cudaStream_t st, int parity)
 int PlainPlan::enqueue_vpass(cudaStream_t st, int parity)
 {
     const int vgrid = (int)((n + vpass_rows - 1) / vpass_rows);
-    pick_vpass(vpass_rows, vpass_staged)<<<vgrid, vpass_threads, vpass_smem, st>>>(v_w, ldv, (int)n,
-                                                                                    parity ? cs2 : cs, rounds, npairs);
+    const int slots = (npairs + vpass_threads - 1) / vpass_threads;
+    pick_vpass(vpass_rows, vpass_staged, slots)<<<vgrid, vpass_threads, vpass_smem, st>>>(
+        v_w, ldv, (int)n, parity ? cs2 : cs, rounds, npairs);
     JSVD_CUDA_TRY(cudaGetLastError());
     return JSVD_OK;
 }
@@ -850,7 +1204,7 @@ int PlainPlan::gram_converged(cudaStream_t st, bool &converged)
         JSVD_CUDA_TRY(cudaMallocHost((void **)&h_gram_count, sizeof(unsigned)));
         JSVD_CUDA_TRY(cudaStreamSynchronize(stream));
     }
-    if (const int rc = dgemm(st, 'T', 'N', (int)n, (int)n, (int)m, 1.0, a_w, lda, a_w, lda, 0.0, gram, (long)n, 1);
+    if (const int rc = dgemm(st, 'T', 'N', (int)n, (int)n, (int)m, 1.0, a_cur, lda, a_cur, lda, 0.0, gram, (long)n, 1);
         rc != JSVD_OK)
         return rc;
     JSVD_CUDA_TRY(cudaMemsetAsync(gram_count, 0, sizeof(unsigned), st));
@@ -872,6 +1226,7 @@ int PlainPlan::run(const double *d_a, double *out_u, double *out_sigma, double *
 
     PlainStats &st = plain_stats();
     int executed = 0;
+    a_cur = a_w;
     if (rounds == 0) {
         executed = 1;  // n == 1: one empty sweep, as the reference reports
     } else {
@@ -960,9 +1315,11 @@ int PlainPlan::run(const double *d_a, double *out_u, double *out_sigma, double *
                 return JSVD_ERR_RUNTIME;
             }
             executed = s + 1;
+            // a sweep of an odd number of fused launches ends in the other copy
+            if (fused_rounds > 0 && (fused_launches() & 1)) a_cur = p ? a_w : a_w2;
             float r_ms = 0.f;
             if (cudaEventElapsedTime(&r_ms, ev_round_begin, ev_round_end) == cudaSuccess) st.round_ms += r_ms;
-            st.round_launches += (unsigned long long)rounds;
+            st.round_launches += (unsigned long long)sweep_launches();
             if (rotated == 0) break;  // V unchanged by this sweep: no V pass
             // The V pass of sweep s runs on vstream while the rounds of sweep
             // s + 1 run on `stream`; the (c, s) tables alternate between
@@ -1000,12 +1357,12 @@ int PlainPlan::run(const double *d_a, double *out_u, double *out_sigma, double *
     st.sweeps += (unsigned long long)executed;
     st.other_launches += 2 + rowmajor_to_colmajor_launches(im) + (out_u ? 1 : 0) + (out_v ? 1 : 0);
     double *sig = out_sigma ? out_sigma : sigma_w;
-    pick_sigma(T)<<<in, T, 0, stream>>>(a_w, lda, im, sig);
+    pick_sigma(T)<<<in, T, 0, stream>>>(a_cur, lda, im, sig);
     JSVD_CUDA_TRY(cudaGetLastError());
     dim3 block(kTile, kTileRows);
     if (out_u) {
         dim3 grid((im + kTile - 1) / kTile, (in + kTile - 1) / kTile);
-        colmajor_to_rowmajor_kernel<<<grid, block, 0, stream>>>(a_w, lda, im, in, out_u, sig, eps);
+        colmajor_to_rowmajor_kernel<<<grid, block, 0, stream>>>(a_cur, lda, im, in, out_u, sig, eps);
         JSVD_CUDA_TRY(cudaGetLastError());
     }
     if (out_v) {

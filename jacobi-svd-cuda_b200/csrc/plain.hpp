@@ -37,6 +37,8 @@ struct PlainPlan {
     size_t bytes = 0;
 
     double *a_w = nullptr;      // column-major working copy of A (m x n)
+    double *a_w2 = nullptr;     // second copy of A: fused launches read one and write the other
+    double *a_cur = nullptr;    // the copy that holds A after the last sweep of a run
     double *v_w = nullptr;      // column-major V (n x n)
     double *sigma_w = nullptr;  // sigma when the caller does not want it
     int2 *pairs = nullptr;      // rounds x npairs schedule
@@ -44,6 +46,10 @@ struct PlainPlan {
     double2 *cs2 = nullptr;     // (c, s) of every pair of odd sweeps
     unsigned *counter = nullptr;  // [0] rotations in the sweep, [1] device status
     int *flags = nullptr;         // persistent sweep: rounds completed per CTA
+    int fused_rounds = 0;         // rounds per launch (0: the one-round kernel)
+    int fused_slots = 0;          // pair slots per CTA of the fused kernel
+    int fused_launches() const { return (rounds + fused_rounds - 1) / fused_rounds; }  // per sweep
+    int sweep_launches() const { return fused_rounds > 0 ? fused_launches() : rounds; }
     bool persistent = false;      // one cooperative launch per sweep
     int slots_per_cta = 1, sweep_grid = 0;
     int mode = 0;         // sweep_mode() at creation
@@ -99,9 +105,10 @@ struct PlainStats {
 };
 PlainStats &plain_stats();
 
-// Process-wide choice of how a sweep is launched: 0 = one kernel per round,
-// replayed from a CUDA graph, each CTA reducing the dot products and deriving
-// the angle in one warp (the default), 1 = one persistent cooperative kernel
+// Process-wide choice of how a sweep is launched: 0 = one kernel per round, or per
+// several rounds where that is faster (fused_shape), replayed from a CUDA graph,
+// each CTA reducing the dot products and deriving a pair's angle once (the
+// default), 1 = one persistent cooperative kernel
 // per sweep, 2 = as 0 with programmatic dependent launch between rounds, 3 = as
 // 0 with every warp deriving the angle itself (one barrier fewer).  Plans
 // record the mode they were created with.
