@@ -30,12 +30,14 @@
 #include <vector>
 
 #include "blockpair.hpp"
+#include "common.cuh"
 #include "dgemm.hpp"
 #include "internal.hpp"
 #include "jsvd.h"
 #include "layout.cuh"
 #include "mixed.hpp"
 #include "plain.hpp"
+#include "ptx.cuh"
 
 namespace jsvd {
 namespace {
@@ -88,147 +90,209 @@ __global__ void __launch_bounds__(256) pc_shift_diagonal(double *__restrict__ G,
 // factor into Linv (column-major, ld = kNb).  The block is padded to kNb x kNb
 // with the identity.
 //
-// The factor is computed as G = L D L^T (L unit lower): each column costs one
-// reciprocal of its pivot on the serial chain, and the square roots are taken
-// afterwards, all at once (Cholesky factor L sqrt(D), inverse
-// D^{-1/2} L^{-1}, where L^{-1} needs no division).  Panels of kPanel columns:
-//   factorisation: warp 0 factors the panel's columns (right-looking inside
-//     the panel, __syncwarp between columns; each lane owns two rows and reads
-//     the pivot column's panel entries before they are rescaled), then all
-//     threads apply the panel's update to the trailing triangle,
-//     a[i][k] -= sum_j L(i,j) d_j L(k,j);
-//   inverse of L: block forward substitution of [L | I], kPanel rows at a
-//     time: thread c solves column c through the panel's unit triangle, then
-//     all threads subtract the panel's contribution from the rows below.
-// A form with a square root and a reciprocal per column measured about 60 us
-// per block on B200 (ncu), set by that serial chain of 64 pivots.
+// The factor is computed as G = L D L^T (L unit lower) by eliminating the
+// augmented block [G | I], which leaves L^{-1} in the right half; the square
+// roots come last (Cholesky factor L sqrt(D), inverse D^{-1/2} L^{-1}).  Panels
+// of 8 columns, both halves in shared memory:
+//   * warps 0-1 (a thread per row) and 2-3 (a thread per column of the right
+//     half) each eliminate the panel's 8 x 8 diagonal block in registers,
+//     carrying their own row or column along: nothing is exchanged on the chain
+//     of pivots (a reciprocal and two fused operations each);
+//   * warps 4-11 meanwhile subtract the previous panel's contribution from the
+//     8 x 8 tiles that later panels need (two DMMA per tile), and scale and
+//     write that panel's columns and rows;
+//   * then warps 4-11 bring the next panel's tiles up to date, one tile each.
+// Two barriers per panel.  What bounds it is the chain: 8 pivots per panel, 8
+// panels.  Per block (B200, back to back): 49 us with one warp on each panel's
+// chain and a division of labour by index arithmetic, 22.6 us with one or two
+// columns per step spread over all threads (shared-memory loads and the
+// step's exchange: 560 cycles per column), 18.5 with the tiles in registers
+// (finding the next panel's among them: 1100 cycles per panel), 14.3 now.
 // status <- 1 on a pivot that is not positive and finite.
-constexpr int kPanel = 8;
-constexpr int kDiagThreads = 256;
-constexpr size_t kDiagSmem = sizeof(double) * 2 * kNb * (kNb + 1);
+constexpr int kDiagThreads = 384;
 
-__global__ void __launch_bounds__(kDiagThreads) pc_chol_inv_diag(const double *__restrict__ G,
-                                                                 double *__restrict__ Lm, int n, int k0, int kb,
-                                                                 double *__restrict__ Linv, int *__restrict__ status)
+// 1 / d for a pivot d: from the hardware's approximation r (relative error
+// e = 1 - d r of about 2^-20) as r (1 + e + e^2).  A pivot outside the
+// approximation's range is divided by; one that is not positive and finite is
+// replaced by 1 and clears ok.
+__device__ __noinline__ double pc_reciprocal_rare(double &d, bool &ok)
 {
-    extern __shared__ double dsm[];
-    __shared__ double dvec[kNb];  // pivots d_i
-    __shared__ double sq[kNb];    // sqrt(d_i)
-    __shared__ double isq[kNb];   // 1 / sqrt(d_i)
-    double(*a)[kNb + 1] = reinterpret_cast<double(*)[kNb + 1]>(dsm);
-    double(*x)[kNb + 1] = reinterpret_cast<double(*)[kNb + 1]>(dsm + kNb * (kNb + 1));
-    const int t = threadIdx.x;
+    if (!(d > 0.0 && d < INFINITY)) {
+        ok = false;
+        d = 1.0;
+    }
+    return 1.0 / d;
+}
+
+__device__ __forceinline__ double pc_reciprocal(double &d, bool &ok)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-d, r, 1.0);
+    r = fma(r, fma(e, e, e), r);
+    const unsigned hi = (unsigned)__double2hiint(d);  // 2^-1000 <= d < 2^1000
+    if (hi - 0x01700000u >= 0x7e700000u - 0x01700000u) r = pc_reciprocal_rare(d, ok);
+    return r;
+}
+
+constexpr int kDiagP = 8;                // columns per panel
+constexpr int kDiagM = kNb + 2;          // row stride of the halves (16-byte row reads without bank conflicts)
+constexpr int kDiagL = 12, kDiagX = kNb + 4;  // row strides of the panel's buffers (DMMA fragment reads likewise)
+constexpr size_t kDiagSmem =
+    sizeof(double) * (2 * kNb * kDiagM + 4 * kNb * kDiagL + 2 * kDiagP * kDiagX + 2 * kDiagP);
+
+__global__ void __launch_bounds__(kDiagThreads, 1) pc_chol_inv_diag(const double *__restrict__ G,
+                                                                    double *__restrict__ Lm, int n, int k0, int kb,
+                                                                    double *__restrict__ Linv,
+                                                                    int *__restrict__ status)
+{
+    constexpr int kP = kDiagP, kPanels = kNb / kP;
+    extern __shared__ __align__(16) double dsm[];
+    double(*A)[kDiagM] = reinterpret_cast<double(*)[kDiagM]>(dsm);  // left half (lower tiles), right half
+    double(*X)[kDiagM] = A + kNb;
+    double(*lp)[kNb][kDiagL] = reinterpret_cast<double(*)[kNb][kDiagL]>(X + kNb);  // L of the panel, by its parity
+    double(*ld)[kNb][kDiagL] = lp + 2;                                             // L D of the panel
+    double(*xo)[kP][kDiagX] = reinterpret_cast<double(*)[kP][kDiagX]>(ld + 2);     // its rows of L^{-1}
+    double(*dv)[kP] = reinterpret_cast<double(*)[kP]>(xo + 2);                     // its pivots
+    __shared__ double sq[kP], isq[kP];
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     {
-        // all of a thread's loads in flight before its stores
-        constexpr int kPer = kNb * kNb / kDiagThreads;
-        double g[kPer];
+        constexpr int kIt = (kNb * kNb + kDiagThreads - 1) / kDiagThreads;
+        double g[kIt];
 #pragma unroll
-        for (int u = 0; u < kPer; ++u) {
-            const int e = t + u * kDiagThreads;
-            const int i = e % kNb, k = e / kNb;  // consecutive threads read consecutive rows of column k
+        for (int u = 0; u < kIt; ++u) {
+            const int e = t + u * kDiagThreads, i = e & (kNb - 1), k = e >> 6;
             g[u] = (i < kb && k < kb) ? (i >= k ? G[(size_t)(k0 + k) * n + k0 + i] : 0.0) : (i == k ? 1.0 : 0.0);
         }
 #pragma unroll
-        for (int u = 0; u < kPer; ++u) {
-            const int e = t + u * kDiagThreads;
-            const int i = e % kNb, k = e / kNb;
-            a[i][k] = g[u];
-            x[i][k] = (i == k) ? 1.0 : 0.0;
+        for (int u = 0; u < kIt; ++u) {
+            const int e = t + u * kDiagThreads, i = e & (kNb - 1), k = e >> 6;
+            if (e < kNb * kNb) {
+                A[i][k] = g[u];
+                X[i][k] = i == k ? 1.0 : 0.0;
+            }
         }
     }
     __syncthreads();
-    // ---- G = L D L^T ----
-    for (int c0 = 0; c0 < kNb; c0 += kPanel) {
-        if (t < 32) {
-            const int lane = t;
-            for (int j = 0; j < kPanel; ++j) {
-                const int cj = c0 + j;
-                const double d0 = a[cj][cj];
-                const bool ok = d0 > 0.0 && d0 < INFINITY;
-                const double d = ok ? d0 : 1.0;
-                // 1 / d by Newton's iteration r <- r (2 - d r) from the
-                // single-precision reciprocal (2^-23 -> 2^-46 -> rounding),
-                // by division outside the single-precision range
-                double rd;
-                if (d > 1.0e-30 && d < 1.0e30) {
-                    rd = (double)__frcp_rn((float)d);
-                    rd = rd * fma(-d, rd, 2.0);
-                    rd = rd * fma(-d, rd, 2.0);
+    if (warp < 4) {
+        const bool rows = warp < 2;
+        const int i = t & (kNb - 1);
+        for (int p = 0; p < kPanels; ++p) {
+            const int b = p & 1, j0 = kP * p;
+            // the diagonal block (lower triangle) and this thread's row of the
+            // panel (warps 0-1) or column of the right half (warps 2-3)
+            double d8[kP][kP], v[kP];
+#pragma unroll
+            for (int r = 0; r < kP; ++r)
+#pragma unroll
+                for (int q = 0; q <= r; q += 2) {
+                    const double2 w = *reinterpret_cast<const double2 *>(&A[j0 + r][j0 + q]);
+                    d8[r][q] = w.x;
+                    if (q + 1 <= r) d8[r][q + 1] = w.y;
+                }
+            if (rows) {
+#pragma unroll
+                for (int j = 0; j < kP; j += 2) {
+                    const double2 w = *reinterpret_cast<const double2 *>(&A[i][j0 + j]);
+                    v[j] = w.x;
+                    v[j + 1] = w.y;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < kP; ++j) v[j] = X[j0 + j][i];
+            }
+            double *lrow = lp[b][i], *drow = ld[b][i];
+            bool ok = true;
+#pragma unroll
+            for (int j = 0; j < kP; ++j) {
+                double d = d8[j][j];
+                const double rd = pc_reciprocal(d, ok);
+                if (t == 0) dv[b][j] = d;
+                double l[kP];
+#pragma unroll
+                for (int r = j + 1; r < kP; ++r) {
+                    l[r] = d8[r][j] * rd;
+#pragma unroll
+                    for (int q = j + 1; q <= r; ++q) d8[r][q] = fma(-l[r], d8[q][j], d8[r][q]);
+                }
+                if (rows) {
+                    const double lv = v[j] * rd;
+                    drow[j] = v[j];
+                    lrow[j] = i > j0 + j ? lv : 0.0;
+#pragma unroll
+                    for (int q = j + 1; q < kP; ++q) v[q] = fma(-lv, d8[q][j], v[q]);
                 } else {
-                    rd = 1.0 / d;
+#pragma unroll
+                    for (int r = j + 1; r < kP; ++r) v[r] = fma(-l[r], v[j], v[r]);
                 }
-                if (lane == 0) {
-                    if (!ok) atomicExch(status, 1);
-                    dvec[cj] = d;
-                }
-                double colk[kPanel];  // a[k][cj] = L(k,cj) d_cj of the panel rows below cj
+            }
+            if (!rows) {
 #pragma unroll
-                for (int kk = 0; kk < kPanel; ++kk) colk[kk] = (kk > j) ? a[c0 + kk][cj] : 0.0;
-                __syncwarp();
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int i = c0 + lane + 32 * h;
-                    if (i >= kNb || i <= cj) continue;
-                    const double lij = a[i][cj] * rd;
-                    a[i][cj] = lij;
-#pragma unroll
-                    for (int kk = 0; kk < kPanel; ++kk) {
-                        const int k = c0 + kk;
-                        if (kk > j && k <= i) a[i][k] = fma(-lij, colk[kk], a[i][k]);
+                for (int j = 0; j < kP; ++j) xo[b][j][i] = v[j];
+            }
+            if (t == 0 && !ok) atomicExch(status, 1);
+            __syncthreads();                       // the panel is eliminated
+            if (p + 1 < kPanels) __syncthreads();  // the next one is up to date
+        }
+    } else {
+        const int fr = lane >> 2, fk = lane & 3, s = t - 128, w = warp - 4;
+        // tile (i, c) of one half less panel p's contribution
+        auto update = [&](int p, int i, int c, bool right) {
+            const int b = p & 1;
+            double2 *C = reinterpret_cast<double2 *>(right ? &X[8 * i + fr][8 * c + 2 * fk]
+                                                           : &A[8 * i + fr][8 * c + 2 * fk]);
+            const double *l = lp[b][8 * i + fr];
+            const double a0 = -l[fk], a1 = -l[4 + fk];
+            const double b0 = right ? xo[b][fk][8 * c + fr] : ld[b][8 * c + fr][fk];
+            const double b1 = right ? xo[b][4 + fk][8 * c + fr] : ld[b][8 * c + fr][4 + fk];
+            const double2 old = *C;
+            double acc[2] = {old.x, old.y};
+            dmma_m8n8k4(acc, a0, b0);
+            dmma_m8n8k4(acc, a1, b1);
+            *C = make_double2(acc[0], acc[1]);
+        };
+        // panel p's columns of the factor and rows of the inverse
+        auto write_out = [&](int p) {
+            const int b = p & 1;
+            if (s < kP) {
+                const double r = sqrt(dv[b][s]);
+                sq[s] = r;
+                isq[s] = 1.0 / r;
+            }
+            group_barrier(1, kDiagThreads - 128);
+            for (int e = s; e < kP * kNb; e += kDiagThreads - 128) {
+                const int i = e & (kNb - 1), j = e >> 6, k = kP * p + j;  // L(i, k)
+                if (i >= k && i < kb) Lm[(size_t)(k0 + k) * n + k0 + i] = (i == k) ? sq[j] : lp[b][i][j] * sq[j];
+                const int r = e & (kP - 1), c = e >> 3, row = kP * p + r;  // L^{-1}(row, c)
+                Linv[row + (size_t)c * kNb] = (row < kb && c <= row) ? xo[b][r][c] * isq[r] : 0.0;
+            }
+        };
+        for (int p = 0; p < kPanels; ++p) {
+            if (p > 0) {
+                // panel p - 1's contribution to the rows below panel p: left
+                // half columns right of p, right half columns up to p - 1 (the
+                // others' rows of L^{-1} are zero)
+                int e = w;
+                for (int i = p + 1; i < kPanels; ++i) {
+                    const int left = i - p;
+                    for (; e < left + p; e += 8) {
+                        const bool right = e >= left;
+                        update(p - 1, i, right ? e - left : p + 1 + e, right);
                     }
+                    e -= left + p;
                 }
-                __syncwarp();
+                write_out(p - 1);
+            }
+            __syncthreads();
+            if (p + 1 < kPanels) {
+                // the next panel: left half rows p + 1 .. 7 of its column,
+                // right half columns 0 .. p of its row
+                const bool right = w > 6 - p;
+                update(p, right ? p + 1 : p + 1 + w, right ? w - (7 - p) : p + 1, right);
+                __syncthreads();
             }
         }
-        __syncthreads();
-        const int base = c0 + kPanel, w = kNb - base;
-        for (int e = t; e < w * w; e += kDiagThreads) {
-            const int i = base + e / w, k = base + e % w;
-            if (k > i) continue;
-            double acc = a[i][k];
-#pragma unroll
-            for (int jj = 0; jj < kPanel; ++jj) acc = fma(-a[i][c0 + jj], a[k][c0 + jj] * dvec[c0 + jj], acc);
-            a[i][k] = acc;
-        }
-        __syncthreads();
-    }
-    if (t < kNb) {
-        sq[t] = sqrt(dvec[t]);
-        isq[t] = 1.0 / sq[t];
-    }
-    // ---- L^{-1}: forward substitution of [L | I] (unit diagonal) ----
-    for (int r0 = 0; r0 < kNb; r0 += kPanel) {
-        const int cols = r0 + kPanel;  // columns 0 .. cols-1 can be non-zero in these rows
-        if (t < cols) {
-            const int c = t;
-#pragma unroll
-            for (int r = 0; r < kPanel; ++r) {
-                const int i = r0 + r;
-                double val = x[i][c];
-#pragma unroll
-                for (int rr = 0; rr < r; ++rr) val = fma(-a[i][r0 + rr], x[r0 + rr][c], val);
-                x[i][c] = val;
-            }
-        }
-        __syncthreads();
-        const int below = kNb - cols;
-        for (int e = t; e < below * cols; e += kDiagThreads) {
-            const int i = cols + e / cols, c = e % cols;
-            double acc = x[i][c];
-#pragma unroll
-            for (int r = 0; r < kPanel; ++r) acc = fma(-a[i][r0 + r], x[r0 + r][c], acc);
-            x[i][c] = acc;
-        }
-        __syncthreads();
-    }
-    // Cholesky factor L sqrt(D) and its inverse D^{-1/2} L^{-1}
-    for (int e = t; e < kb * kb; e += kDiagThreads) {
-        const int i = e % kb, k = e / kb;
-        if (i >= k) Lm[(size_t)(k0 + k) * n + k0 + i] = (i == k) ? sq[i] : a[i][k] * sq[k];
-    }
-    for (int e = t; e < kNb * kNb; e += kDiagThreads) {
-        const int i = e % kNb, k = e / kNb;
-        Linv[i + (size_t)k * kNb] = (i < kb && k < kb && k <= i) ? x[i][k] * isq[i] : 0.0;
+        write_out(kPanels - 1);
     }
 }
 
@@ -381,7 +445,6 @@ int acquire_pc_plan(int dev, size_t m, size_t n, size_t ws_doubles, PcPlan **out
     }
     JSVD_CUDA_TRY(cudaMallocAsync((void **)&p->ws, sizeof(double) * ws_doubles, p->own));
     JSVD_CUDA_TRY(cudaStreamSynchronize(p->own));
-    JSVD_CUDA_TRY(cudaFuncSetAttribute(pc_chol_inv_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem));
     plans.insert(plans.begin(), std::move(p));
     while (plans.size() > kPcMaxPlans) plans.pop_back();
     *out = plans.front().get();
