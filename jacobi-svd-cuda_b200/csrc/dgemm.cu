@@ -127,19 +127,40 @@ __global__ void __launch_bounds__((BM / 32) * (BN / 32) * 32)
         }
     }
     cp_async_wait<0>();
+    // C's old values are all loaded before any store: a load cannot pass a
+    // store to the same array, so one element at a time the epilogue was a chain
+    // of 32 loads (a 64 x 64 x 64 product with beta = 1: 20 us, with beta = 0:
+    // 7.6 us, alone on the device).
+    // The 128-row tile has registers for half of them at a time.
+    constexpr int kHold = BM >= 128 ? 2 : 4;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int row = m0 + wm * 32 + i * 8 + fr;
-        if (row >= m) continue;
+    for (int i0 = 0; i0 < 4; i0 += kHold) {
+        double old[kHold][4][2];
+        if (beta != 0.0) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+            for (int i = 0; i < kHold; ++i)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int col = n0 + wn * 32 + j * 8 + 2 * fk + h;
-                if (col >= n || (lower && col > row)) continue;
-                double *cp = C + (size_t)row + (size_t)col * ldc;
-                const double v = alpha * acc[i][j][h];
-                *cp = (beta == 0.0) ? v : fma(beta, *cp, v);
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int row = m0 + wm * 32 + (i0 + i) * 8 + fr, col = n0 + wn * 32 + j * 8 + 2 * fk + h;
+                        const bool live = row < m && col < n && !(lower && col > row);
+                        old[i][j][h] = live ? C[(size_t)row + (size_t)col * ldc] : 0.0;
+                    }
+        }
+#pragma unroll
+        for (int i = 0; i < kHold; ++i) {
+            const int row = m0 + wm * 32 + (i0 + i) * 8 + fr;
+            if (row >= m) continue;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int col = n0 + wn * 32 + j * 8 + 2 * fk + h;
+                    if (col >= n || (lower && col > row)) continue;
+                    const double v = alpha * acc[i0 + i][j][h];
+                    C[(size_t)row + (size_t)col * ldc] = (beta == 0.0) ? v : fma(beta, old[i][j][h], v);
+                }
             }
         }
     }
