@@ -107,6 +107,27 @@ __device__ __forceinline__ void group_barrier(int id, int threads)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Arrives at that barrier without waiting.
+__device__ __forceinline__ void group_barrier_arrive(int id, int threads)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// 1 / d to about one ulp for 2^-1000 <= d < 2^1000 (reciprocal_in_range), from
+// the hardware's approximation r (relative error e = 1 - d r of about 2^-20) as
+// r (1 + e + e^2).
+__device__ __forceinline__ bool reciprocal_in_range(double d)
+{
+    return (unsigned)__double2hiint(d) - 0x01700000u < 0x7e700000u - 0x01700000u;
+}
+__device__ __forceinline__ double approx_reciprocal(double d)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // Rutishauser rotation for the 2x2 Gram [pp pq; pq qq]; returns true when the
 // pair rotates.  A pair that does not rotate reports c = 0, s = 0 (a real
 // rotation always has c >= 1/sqrt(2)), which is how the deferred V update

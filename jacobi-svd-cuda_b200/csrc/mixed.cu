@@ -41,6 +41,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -78,11 +79,16 @@ __device__ __forceinline__ uint8_t *align1024(uint8_t *p)
 __device__ __forceinline__ void record_status(int *status, int code) { atomicCAS(status, 0, code); }
 
 // Partial Gram of block pair blockIdx.y over row chunks [c0, c1) (32 rows
-// each) of split blockIdx.x.  Output: the raw 128 x 64 FP32 accumulator,
-// column-major, at part + (pair * splits + split) * 8192.
+// each) of split blockIdx.x.  Output: the upper triangle of the 64 x 64 Gram in
+// FP64, column-major, at part + (pair * splits + split) * 4096: D[0:64] +
+// D[64:128], the mean of the two triangles (they come from different
+// accumulation orders).  Converted here, by the many CTAs of this kernel, and
+// not by the eigen-solve's one CTA per pair, whose set-up it bounded (65,536
+// conversions at 16 per cycle; with putting the triangles together 14,400
+// cycles of that CTA, 6,600 now, at 1 us more here).
 __global__ void __launch_bounds__(kGramTcThreads)
     mx_gram_tc(const __grid_constant__ CUtensorMap mh, const __grid_constant__ CUtensorMap ml, int nb, int round,
-               int kchunks, int chunks_per_split, float *__restrict__ part, int *__restrict__ status)
+               int kchunks, int chunks_per_split, double *__restrict__ part, int *__restrict__ status)
 {
     extern __shared__ uint8_t smraw[];
     uint8_t *sm = align1024(smraw);
@@ -159,21 +165,31 @@ __global__ void __launch_bounds__(kGramTcThreads)
         __syncwarp();
     }
     if (warp < 4) {
-        const bool ok = mbar_wait(accf, 0);
+        // a wait that ran out is recorded; the epilogue's barriers are passed all
+        // the same (its values are then not used)
+        if (!mbar_wait(accf, 0)) record_status(status, kDevWaitTimeout);
         tc_fence_after();
-        if (!ok) {
-            record_status(status, kDevWaitTimeout);
-        } else {
-            float *out = part + ((size_t)pair * gridDim.x + split) * (128 * 64);
-            const int r = warp * 32 + lane;
-            float v[32];
+        // the operand stages are free: the rows to be added as FP32, then the sums
+        float *lo = reinterpret_cast<float *>(tiles);                   // [64 columns][64 rows]
+        double *sum = reinterpret_cast<double *>(tiles + kW * kW * 4);  // [64 columns][65]
+        // (each half of the rows adds up one half of the columns)
+        const int r = (warp & 1) * 32 + lane, mine = (warp >> 1) * 32, other = 32 - mine;
+        const uint32_t src = tmem + ((uint32_t)(warp * 32) << 16);
+        float v[32];
+        tmem_ld32(src + other, v);
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + half * 32, v);
+        for (int c = 0; c < 32; ++c) lo[(other + c) * kW + r] = v[c];
+        tmem_ld32(src + mine, v);
+        group_barrier(1, 128);
 #pragma unroll
-                for (int c = 0; c < 32; ++c) out[(size_t)(half * 32 + c) * 128 + r] = v[c];
-            }
-        }
+        for (int c = 0; c < 32; ++c)
+            sum[(mine + c) * (kW + 1) + r] = (double)v[c] + (double)lo[(mine + c) * kW + r];
+        group_barrier(1, 128);
+        double *out = part + ((size_t)pair * gridDim.x + split) * (kW * kW);
+        const int row = threadIdx.x & (kW - 1);
+#pragma unroll 8
+        for (int c = threadIdx.x >> 6; c < kW; c += 2)
+            if (row <= c) out[c * kW + row] = 0.5 * (sum[c * (kW + 1) + row] + sum[row * (kW + 1) + c]);
     }
     tc_fence_before();
     __syncthreads();
@@ -500,108 +516,24 @@ __global__ void __launch_bounds__(kRot64Threads)
 // Block eigen-solve (FP64, both phases)
 // ============================================================================
 
-constexpr int kEvdThreads = 512;      // warps 0-7: W (and 48 blocks of G); warps 8-14: G; warp 15: the angles
-constexpr int kEvdWThreads = 256;     // a warp per (half of the rows, quarter of the slots) of W
-constexpr int kEvdBulkThreads = 224;  // warps 8-14
+// Warp roles.  A warp's scheduler is its id mod 4 (its FP64 pipe too): the
+// angle warp has one to itself, the other roles take the warps of the other
+// three (bulk index 0 .. 17), and the rest of its scheduler's warps only help
+// to set up.  Bulk 0-7: W, a warp per (half of the rows, quarter of the slots);
+// bulk 8-15: G, two groups of 32 blocks each.
+constexpr int kEvdWarps = 24, kEvdThreads = 32 * kEvdWarps;
+constexpr int kEvdAngleWarp = 3, kEvdW = 8, kEvdBulk = 16;
+constexpr int kEvdBulkIters = 2;  // blocks per G thread
+constexpr int kEvdLoopThreads = 32 * (kEvdBulk + 1);  // threads of the round loop
 constexpr int kEvdQ = kW / 2 + 1;     // row stride of a quadrant of G (odd: column accesses hit distinct banks)
 constexpr int kEvdQuad = (kW / 2) * kEvdQ;  // one 32 x 33 quadrant
 constexpr int kEvdG = 3 * kEvdQuad;   // G: first-first, first-second, second-second quadrants
-constexpr int kEvdTmpLD = kW + 1;     // the input Gram in column coordinates (set-up only)
+constexpr int kEvdWLD = kW + 1;       // W on its way out: [column][row]
 constexpr int kOffBlocks = (kW / 2) * (kW / 2 - 1) / 2;  // 2x2 blocks (a < b) of the 32 x 32 block grid
-constexpr int kEvdBulkIters = 2;      // blocks per G thread (the last 48 go to W threads 0-47)
 constexpr int kEvdRounds = kW - 1;
 constexpr int kEvdMaxInner = 8;
-constexpr size_t kEvdSmem = sizeof(double) * (kEvdG + kW * kEvdTmpLD);  // G0, then G1 / the set-up buffer
-static_assert(kOffBlocks - kEvdBulkIters * kEvdBulkThreads <= kEvdWThreads, "G blocks left for the W warps");
-
-// Rotation of [pp pq; pq qq] that annihilates pq, with the reference's
-// threshold test (|pq| > tau sqrt(pp qq), squared, and |pq| > 1e-300), in
-// two parts: evd_prepare takes what depends on the diagonal only (known a
-// round ahead), evd_rotation the rest once pq is known.
-//   t = tan(theta), the smaller root of t^2 + 2 zeta t - 1 = 0 with
-//   zeta = (qq - pp) / (2 pq) (Rutishauser's choice), c = 1 / sqrt(1 + t^2),
-//   s = t c, sign(t) = sign(e) for d = qq - pp >= 0 and -sign(e) otherwise
-//   (e = 2 pq).
-// Small angles (x = |e| / (2 |d|) <= 2^-6): t = (sqrt(1 + 4x^2) - 1) / (2x)
-// = x - x^3 + 2x^5 - 5x^7 + 14x^9 - ... (Catalan-number coefficients) and
-// c = (1 + t^2)^(-1/2) = 1 - z/2 + 3z^2/8 - 5z^3/16 + 35z^4/128 - ...
-// (z = t^2): the terms left out are below 2^-54 relative, so both series,
-// evaluated by Horner's rule from the precomputed 1 / (2 |d|), are exact to
-// rounding: ten fused operations and no square root or division.  Called by
-// a full warp; the path is chosen for the whole warp.  Otherwise, with rho = 1 / sqrt(d^2 + e^2), cos 2theta =
-// |d| rho and sin 2theta = |e| rho, and the half-angle identities give
-//   c^2 = (1 + cos 2theta) / 2 in [1/2, 1],  c = c^2 / sqrt(c^2),
-//   |s| = sin 2theta / (2c),  |t| = |s| / c:
-// two reciprocal square roots, no cancellation; d and e are scaled by a
-// power of two when their magnitude could over- or underflow d^2 + e^2.
-struct EvdPre {
-    double d;    // qq - pp
-    double thr;  // tau^2 max(pp, 0) max(qq, 0)
-    double r2;   // 1 / (2 |d|) (infinite for d = 0), to about one ulp
-};
-
-__device__ __forceinline__ EvdPre evd_prepare(double pp, double qq, double tau)
-{
-    EvdPre p;
-    p.d = qq - pp;
-    p.thr = (tau * tau) * (fmax(pp, 0.0) * fmax(qq, 0.0));
-    // 1 / (2 |d|) by Newton's iteration r <- r (2 - |d| r) from a
-    // single-precision reciprocal (two steps: 2^-23 -> 2^-46 -> rounding);
-    // outside the single-precision range, by division
-    const double ad = fabs(p.d);
-    if (ad > 1.0e-30 && ad < 1.0e30) {
-        double r = (double)__frcp_rn((float)ad);
-        r = r * fma(-ad, r, 2.0);
-        r = r * fma(-ad, r, 2.0);
-        p.r2 = 0.5 * r;
-    } else {
-        p.r2 = 0.5 / ad;
-    }
-    return p;
-}
-
-__device__ __forceinline__ bool evd_rotation(const EvdPre &p, double pq, double &c, double &s, double &t)
-{
-    const bool rot = fabs(pq) > 1.0e-300 && pq * pq > p.thr;
-    double d = p.d, e = 2.0 * pq;
-    const double sg = ((d >= 0.0) == (e >= 0.0)) ? 1.0 : -1.0;
-    const double x = fabs(e) * p.r2;
-    double ta, ca, sa;
-    // one path for the whole warp (the caller's 32 lanes are all active): the
-    // series when every rotating lane's angle is small, else the exact form
-    if (__all_sync(0xffffffffu, x <= 0x1p-6 || !rot)) {
-        const double y = x * x;
-        double p = fma(14.0, y, -5.0);
-        p = fma(p, y, 2.0);
-        p = fma(p, y, -1.0);
-        p = fma(p, y, 1.0);
-        ta = x * p;
-        const double z = ta * ta;
-        double q = fma(35.0 / 128.0, z, -5.0 / 16.0);
-        q = fma(q, z, 3.0 / 8.0);
-        q = fma(q, z, -0.5);
-        ca = fma(q, z, 1.0);
-        sa = ta * ca;
-    } else {
-        const double f = fmax(fabs(d), fabs(e));
-        if (rot && (f > 1.0e150 || f < 1.0e-150)) {
-            const int k = ilogb(f);
-            d = scalbn(d, -k);
-            e = scalbn(e, -k);
-        }
-        const double rho = rsqrt(fma(d, d, e * e));
-        const double c2 = fma(0.5 * fabs(d), rho, 0.5);
-        const double hs = (0.5 * fabs(e)) * rho;  // sin 2theta / 2
-        const double rc = rsqrt(c2);              // 1 / c
-        ca = c2 * rc;
-        sa = hs * rc;
-        ta = sa * rc;
-    }
-    c = rot ? ca : 1.0;
-    s = rot ? sg * sa : 0.0;
-    t = rot ? sg * ta : 0.0;
-    return rot;
-}
+constexpr size_t kEvdSmem = sizeof(double) * (2 * kEvdG + kW * kEvdWLD);  // G's two buffers, W on its way out
+static_assert(kOffBlocks <= kEvdBulkIters * 32 * (kEvdBulk - kEvdW), "blocks of G per thread");
 
 // Slots.  The 64 indices of the eigen-solve move through the circle of the
 // round-robin ordering; instead of looking the pairs up per round, every
@@ -613,14 +545,11 @@ __device__ __forceinline__ bool evd_rotation(const EvdPre &p, double pq, double 
 // At the start (and after every full sweep of 63 rounds, the permutation's
 // order) slot 2k holds index k and slot 2k+1 index 63 - k, which is pair k of
 // round 0 of the circle (round_robin_pair).
-__device__ __forceinline__ int evd_slot_column(int slot) { return (slot & 1) ? 63 - (slot >> 1) : (slot >> 1); }
-__device__ __forceinline__ int evd_column_slot(int col) { return col < 32 ? 2 * col : 127 - 2 * col; }
-__device__ __forceinline__ int evd_next_slot(int s)
+__host__ __device__ constexpr int evd_slot_column(int slot) { return (slot & 1) ? 63 - (slot >> 1) : (slot >> 1); }
+__host__ __device__ constexpr int evd_column_slot(int col) { return col < 32 ? 2 * col : 127 - 2 * col; }
+__host__ __device__ constexpr int evd_next_slot(int s)
 {
-    if (s == 0) return 0;
-    if (s == 1) return 2;
-    if (s == 62) return 63;
-    return (s & 1) ? s - 2 : s + 2;
+    return s == 0 ? 0 : (s == 1 ? 2 : (s == 62 ? 63 : ((s & 1) ? s - 2 : s + 2)));
 }
 // G is symmetric; it is kept as three 32 x 33 quadrants indexed by pair:
 // FF[k][l] = G(first k, first l) and SS[k][l] = G(second k, second l) for
@@ -631,67 +560,139 @@ __device__ __forceinline__ int evd_next_slot(int s)
 // circle's ends): with the odd row stride every one of those eight addresses
 // falls in bank (a + b + constant) mod 16, so a warp whose 32 blocks cover
 // each residue of a + b twice accesses G without bank conflicts.
-__device__ __forceinline__ int evd_off(int s, int t)
+__host__ __device__ constexpr int evd_off(int s, int t)
 {
     const int ks = s >> 1, kt = t >> 1;
-    if ((s & 1) == (t & 1)) return ((s & 1) ? 2 * kEvdQuad : 0) + min(ks, kt) * kEvdQ + max(ks, kt);
+    if ((s & 1) == (t & 1)) return ((s & 1) ? 2 * kEvdQuad : 0) + (ks < kt ? ks * kEvdQ + kt : kt * kEvdQ + ks);
     return (s & 1) ? kEvdQuad + kt * kEvdQ + ks : kEvdQuad + ks * kEvdQ + kt;
 }
 
-// The k-th off-diagonal block (a < b) with (a + b) mod 16 == r, in order of
-// a + b, then a.  Residues r even have 30 blocks, odd 32.
-__device__ __forceinline__ int2 evd_block_of(int r, int k)
+// The 496 off-diagonal 2 x 2 blocks in groups of 32 (a G warp's lanes; the last
+// group has 16), in which each half-warp holds every residue of a + b mod 16
+// once (shared memory serves a half-warp's 8-byte accesses per wavefront).  Per
+// block: the pair indices (a | b << 8), the offsets of FF[a][b] (FS[a][b] and
+// SS[a][b] follow at fixed distances) and of FS[b][a], and the destinations of
+// its four entries after the advance, two per int.
+struct EvdBlock {
+    int ab, rof, w01, w23;
+};
+struct EvdBlocks {
+    EvdBlock of[kEvdBulkIters * (kEvdBulk - kEvdW)][32];
+};
+constexpr EvdBlocks evd_make_blocks()
 {
-    for (int d = r; d <= kW - 3; d += 16) {
-        if (d < 1) continue;
-        const int lo = max(0, d - (kW / 2 - 1)), hi = (d - 1) >> 1;
-        const int cnt = hi - lo + 1;
-        if (cnt > 0) {
-            if (k < cnt) return make_int2(lo + k, d - lo - k);
-            k -= cnt;
+    EvdBlocks t{};
+    // by residue of a + b mod 16, in order of a + b, then a: even residues
+    // have 30 blocks, odd ones 32
+    int count[16] = {};
+    for (int sum = 1; sum <= kW - 3; ++sum)
+        for (int a = 0; a < kW / 2; ++a) {
+            const int b = sum - a, res = sum & 15;
+            if (b <= a || b >= kW / 2) continue;
+            const int k = count[res]++;
+            const int g = k < 30 ? k >> 1 : 15;
+            const int lane = k < 30 ? (k & 1) * 16 + res : (k - 30) * 8 + (res >> 1);
+            EvdBlock e{};
+            const int pa = evd_next_slot(2 * a), qa = evd_next_slot(2 * a + 1);
+            const int pb = evd_next_slot(2 * b), qb = evd_next_slot(2 * b + 1);
+            e.ab = a | (b << 8);
+            e.rof = evd_off(2 * a, 2 * b) | (evd_off(2 * a + 1, 2 * b) << 16);
+            e.w01 = evd_off(pa, pb) | (evd_off(pa, qb) << 16);
+            e.w23 = evd_off(qa, pb) | (evd_off(qa, qb) << 16);
+            t.of[g][lane] = e;
         }
-    }
-    return make_int2(-1, -1);
+    return t;
+}
+__device__ const EvdBlocks kEvdBlocks = evd_make_blocks();
+
+// 1 / sqrt(a) to about one ulp for a normal a: one third-order step on the
+// hardware's approximation y (e = 1 - a y^2): y (1 + e / 2 + 3 e^2 / 8).
+__device__ __forceinline__ double approx_rsqrt(double a)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double e = fma(-(a * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
-// W in registers, in slots.  Warp w < 8 holds rows 32 (w & 1) + lane of
-// quarter q = w >> 1 of the slots (pairs 8q .. 8q+7, slots 16q .. 16q+15,
-// local index j <-> pair 8q + j), w[2j] = first, w[2j+1] = second: every
-// lane of a warp applies the same eight rotations (one broadcast load each).
-__device__ __forceinline__ void evd_w_rotate(double (&w)[16], const double2 *cs, int q)
+// Rotation of [pp pq; pq qq] that annihilates pq, with the reference's
+// threshold test (|pq| > tau sqrt(pp qq), squared, and |pq| > 1e-300).
+//   t = tan(theta), the smaller root of t^2 + 2 zeta t - 1 = 0 with
+//   zeta = (qq - pp) / (2 pq) (Rutishauser's choice), c = 1 / sqrt(1 + t^2),
+//   s = t c, sign(t) = sign(e) for d = qq - pp >= 0 and -sign(e) otherwise
+//   (e = 2 pq).
+// With rho = 1 / sqrt(d^2 + e^2), cos 2theta = |d| rho and sin 2theta = |e| rho,
+// and the half-angle identities give
+//   c^2 = (1 + cos 2theta) / 2 in [1/2, 1],  c = c^2 / sqrt(c^2),
+//   |s| = sin 2theta / (2c),  |t| = |s| / c:
+// two reciprocal square roots, no cancellation at any angle; d and e are
+// scaled by a power of two when their magnitude could over- or underflow
+// d^2 + e^2.  It is the chain that bounds a round, and a straight line: a
+// shorter series for small angles, chosen by a vote of the warp, took longer
+// with its vote and branches (246 cycles; 426 for this form behind them).
+__device__ __forceinline__ bool evd_rotation(double pp, double qq, double tau2, double pq, double &c, double &s,
+                                             double &t)
+{
+    const double d = qq - pp;
+    double ad = fabs(d), ae = 2.0 * fabs(pq);
+    // 2^-498 <= max(|d|, |e|) < 2^498 or zero, by the exponent bits
+    const int hi = max(__double2hiint(ad), __double2hiint(ae));
+    if ((unsigned)(hi - 1) < (525u << 20) - 1u || hi >= (1521 << 20)) {
+        const int k = ilogb(fmax(ad, ae));
+        ad = scalbn(ad, -k);
+        ae = scalbn(ae, -k);
+    }
+    const double rho = approx_rsqrt(fma(ad, ad, ae * ae));
+    const double c2 = fma(0.5 * ad, rho, 0.5);
+    const double hs = (0.5 * ae) * rho;  // sin 2theta / 2
+    const double rc = approx_rsqrt(c2);  // 1 / c
+    const double ca = c2 * rc, sa = hs * rc, ta = sa * rc;
+    const double thr = tau2 * (fmax(pp, 0.0) * fmax(qq, 0.0));
+    const bool rot = fabs(pq) > 1.0e-300 && pq * pq > thr;
+    const bool neg = (d >= 0.0) != (pq >= 0.0);
+    c = rot ? ca : 1.0;
+    s = rot ? (neg ? -sa : sa) : 0.0;
+    t = rot ? (neg ? -ta : ta) : 0.0;
+    return rot;
+}
+
+// One quarter row of W: the eight pairs 8q .. 8q+7 of quarter q, rotated by
+// the round's angles and advanced around the circle, in registers that stay
+// put.  Logical pair j's first index is in f[(j - ph) & 7] and its second in
+// s[(j + ph) & 7] at phase ph = round mod 8, so the advance first'[j] =
+// first[j-1], second'[j] = second[j+1] moves nothing; the rounds are unrolled
+// by eight.  The two that cross quarters are kept apart: x0, pair 0's first
+// (the quarter below's last first, through shared memory; the circle's fixed
+// index in quarter 0), and y7, pair 7's second (the quarter above's first
+// second; in quarter 3 its own last first).
+struct EvdRow {
+    double f[8], s[8], x0, y7;
+};
+
+template <int ph>
+__device__ __forceinline__ void evd_w_round(EvdRow &w, const double2 *cs, int q, double &last_first,
+                                            double &first_second)
 {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const double2 r = cs[8 * q + j];
-        const double x = w[2 * j], y = w[2 * j + 1];
-        w[2 * j] = fma(r.x, x, -(r.y * y));
-        w[2 * j + 1] = fma(r.y, x, r.x * y);
+        const double x = j == 0 ? w.x0 : w.f[(j - ph) & 7], y = j == 7 ? w.y7 : w.s[(j + ph) & 7];
+        const double xn = fma(r.x, x, -(r.y * y)), yn = fma(r.y, x, r.x * y);
+        if (j == 0) w.x0 = xn;
+        else w.f[(j - ph) & 7] = xn;
+        if (j == 7) w.y7 = yn;
+        else w.s[(j + ph) & 7] = yn;
     }
+    last_first = w.f[(7 - ph) & 7];
+    first_second = w.s[ph & 7];
+    // pair 1's next first: pair 0's first, in quarter 0 pair 0's second
+    w.f[(0 - ph) & 7] = q == 0 ? first_second : w.x0;
+    // pair 6's next second
+    w.s[(7 + ph) & 7] = w.y7;
 }
 
-// Advance of the circle for one quarter row: up = first[8q - 1] of the
-// quarter below, down = second[8q + 8] of the quarter above (both from the
-// warps holding them, through shared memory).
-__device__ __forceinline__ void evd_w_advance(double (&w)[16], int q, double up, double down)
-{
-    double f[8], s[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        f[j] = w[2 * j];
-        s[j] = w[2 * j + 1];
-    }
-    w[0] = q == 0 ? f[0] : up;
-    w[2] = q == 0 ? s[0] : f[0];
-#pragma unroll
-    for (int j = 2; j < 8; ++j) w[2 * j] = f[j - 1];
-#pragma unroll
-    for (int j = 0; j < 7; ++j) w[2 * j + 1] = s[j + 1];
-    w[15] = q == 3 ? f[7] : down;
-}
-
-// Input Gram of block pair blockIdx.x from `splits` partials: kind 0 = the
-// tensor-core layout (128 x 64 FP32, rows r and r + 64 summed), kind 1 =
-// 64 x 64 FP64 upper triangle.  Cyclic two-sided Jacobi, at most
+// Input Gram of block pair blockIdx.x: the sum of `splits` partials (64 x 64
+// FP64, column-major, upper triangles).  Cyclic two-sided Jacobi, at most
 // inner_sweeps sweeps of 63 rounds of 32 disjoint index pairs, in slot
 // coordinates (above), software pipelined so that a round costs one barrier
 // and the angle chain runs beside the update:
@@ -699,293 +700,289 @@ __device__ __forceinline__ void evd_w_advance(double (&w)[16], int q, double up,
 //     buffer r%2 and writes buffer (r+1)%2 already advanced to round r+1's
 //     slots, so every thread reads and writes the same addresses in every
 //     round (kept in registers, no table lookups);
-//   * warps 8-14 (and threads 0-47) apply round r to the off-diagonal 2 x 2
-//     blocks of slot pairs (a, b), a < b (two 16-byte loads, four stores, the
-//     unrotated blocks copied: c = 1, s = 0 reproduce them);
-//   * warps 0-7 apply it to W (registers; the advance of the circle across
-//     quarters goes through shared memory and completes a round later);
-//   * warp 15 (lane k: pair k) writes the diagonal blocks (the annihilated
-//     pairs) and derives the angles of round r+1 from buffer r%2 and round
-//     r's rotations: pair k of round r+1 takes its first index from pair k-1
-//     of round r (pair 0 for k <= 1) and its second from pair k+1 (pair 31
-//     for k = 31), so its diagonal entries are round r's annihilated
+//   * the G warps apply round r to the off-diagonal 2 x 2 blocks of slot pairs
+//     (a, b), a < b (four loads, four stores each, the unrotated blocks copied:
+//     c = 1, s = 0 reproduce them);
+//   * the W warps apply it to W (evd_w_round);
+//   * the angle warp (lane k: pair k) writes the diagonal blocks (the
+//     annihilated pairs) and derives the angles of round r+1 from buffer r%2
+//     and round r's rotations: pair k of round r+1 takes its first index from
+//     pair k-1 of round r (pair 0 for k <= 1) and its second from pair k+1
+//     (pair 31 for k = 31), so its diagonal entries are round r's annihilated
 //     diagonals and its off-diagonal entry is one element of one 2 x 2 block
 //     update, computed with the same operations as the update itself
-//     (bit-identical to what lands in the buffer).  Everything that depends
-//     on round r's angles only (the new diagonals, the neighbours' angles,
-//     the diagonal part of the rotation) is done before round r's barrier.
+//     (bit-identical to what lands in the buffer).
+// Two paths bound a round, about evenly.  The angle warp's: barrier, loads, four
+// fused operations, the rotation's two reciprocal square roots, publication; it
+// has an FP64 pipe to itself and shares only the shared-memory port (with the
+// other roles on all four schedulers it took 1870 cycles, half of it in
+// queues).  The G warps': shared-memory traffic, 48
+// KB per round, with each thread's loads issued before its stores.  Per round
+// (B200) 1670 cycles before, 950 now; per launch of 16 pairs 67 us, 39-40 now.
 // Writes W (64 x 64, column-major) - and, when Wimg is not null, its 3xTF32
 // operand image for the tensor-core rotation - and flags[pair] = 1 when some
 // pair rotated (else flags[pair] = 0 and W is left as it was).  stats[0] (as
 // double bits) = running max of |g_pq| / sqrt(g_pp g_qq) over the input
 // Grams, stats[1] = number of block pairs that rotated.
 __global__ void __launch_bounds__(kEvdThreads, 1)
-    mx_evd(const void *__restrict__ part, int kind, int splits, double tau, int inner_sweeps, int nb, int round,
+    mx_evd(const double *__restrict__ part, int splits, double tau, int inner_sweeps, int nb, int round,
            int sort, int ncols, double *__restrict__ Wout, float *__restrict__ Wimg, int *__restrict__ flags,
            unsigned long long *__restrict__ stats)
 {
     extern __shared__ __align__(16) double dsm[];
-    double *const G0 = dsm;                 // [64][66], buffer 0
-    double *const G1 = dsm + kEvdG;         // buffer 1 (and, at set-up, the Gram in column coordinates)
+    double *const G0 = dsm;                 // buffer 0
+    double *const G1 = dsm + kEvdG;         // buffer 1
+    double *const Ws = dsm + 2 * kEvdG;
     __shared__ double2 cs[2][kW / 2];       // (c, s) of the 32 pairs, by round parity (W: broadcast loads)
     __shared__ double cs_c[2][kW / 2], cs_s[2][kW / 2];  // the same, apart (G: 8-byte loads of many pairs)
     __shared__ double xf[2][4][kW];         // W advance: first[8q + 7] of quarter q, by row
     __shared__ double xs[2][4][kW];         // W advance: second[8q] of quarter q, by row
-    __shared__ unsigned rot_mask[2];
+    __shared__ double dg[kW];               // the input Gram's diagonal
     __shared__ int sweep_any[kEvdMaxInner + 1];
     __shared__ int out_col[kW];
+    __shared__ int s_rounds;
     __shared__ unsigned long long off_bits;
     const int pair = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int bulk = (warp & 3) == (kEvdAngleWarp & 3) ? kEvdBulk : (warp >> 2) * 3 + (warp & 3);
+    const bool is_angle = warp == kEvdAngleWarp, is_w = bulk < kEvdW, is_g = bulk >= kEvdW && bulk < kEvdBulk;
     const int nsweeps = min(inner_sweeps, kEvdMaxInner);
-    if (tid == 0) off_bits = 0ull;
+    if (tid == 0) {
+        off_bits = 0ull;
+        s_rounds = 0;
+    }
     if (tid <= kEvdMaxInner) sweep_any[tid] = 0;
-    // the input Gram in column coordinates, in buffer 1.  Thread t sums rows
-    // 4j .. 4j+3 of column c for (c, j) = ((t + 512 i) >> 4, (t + 512 i) & 15),
-    // i = 0..1, over the splits: 16-byte loads, four per split in flight
-    // (kind 0 adds rows r and r + 64 of the partial in the same order as the
-    // element-wise sum: g += lo + hi).
-    {
-        constexpr int kI = kW * kW / 4 / kEvdThreads;
-        double acc[kI][4];
+    // the input Gram, summed over the splits (eight in flight), to buffer 0 in
+    // slot coordinates.  A unit is rows 2j, 2j+1 of column c, 2j <= c; columns i
+    // and 63 - i have 33 together
+    constexpr int kUnits = (kW / 2) * (kW / 2 + 1), kI = (kUnits + kEvdThreads - 1) / kEvdThreads;
+    double acc[kI][2];
+    int ucol[kI], urow[kI];
 #pragma unroll
-        for (int i = 0; i < kI; ++i)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) acc[i][k] = 0.0;
-        if (kind == 0) {
-            const float *p = static_cast<const float *>(part) + (size_t)pair * splits * 8192;
-#pragma unroll 4
+    for (int i = 0; i < kI; ++i) {
+        const int u = tid + kEvdThreads * i, fold = u / (kW / 2 + 1), k = u - fold * (kW / 2 + 1);
+        const bool second = k > fold / 2;
+        ucol[i] = u < kUnits ? (second ? kW - 1 - fold : fold) : -1;
+        urow[i] = 2 * (second ? k - fold / 2 - 1 : k);
+        acc[i][0] = acc[i][1] = 0.0;
+        if (ucol[i] >= 0) {
+            const double *p = part + (size_t)pair * splits * (kW * kW) + ucol[i] * kW + urow[i];
+#pragma unroll 8
             for (int s = 0; s < splits; ++s) {
-                float4 lo[kI], hi[kI];
-#pragma unroll
-                for (int i = 0; i < kI; ++i) {
-                    const int o = tid + kEvdThreads * i, c = o >> 4, j = o & 15;
-                    const float *q = p + (size_t)s * 8192 + c * 128 + 4 * j;
-                    lo[i] = __ldg(reinterpret_cast<const float4 *>(q));
-                    hi[i] = __ldg(reinterpret_cast<const float4 *>(q + 64));
-                }
-#pragma unroll
-                for (int i = 0; i < kI; ++i) {
-                    acc[i][0] += (double)lo[i].x + (double)hi[i].x;
-                    acc[i][1] += (double)lo[i].y + (double)hi[i].y;
-                    acc[i][2] += (double)lo[i].z + (double)hi[i].z;
-                    acc[i][3] += (double)lo[i].w + (double)hi[i].w;
-                }
+                const double2 v = __ldg(reinterpret_cast<const double2 *>(p + (size_t)s * (kW * kW)));
+                acc[i][0] += v.x;
+                acc[i][1] += v.y;
             }
-        } else {
-            const double *p = static_cast<const double *>(part) + (size_t)pair * splits * 4096;
-#pragma unroll 4
-            for (int s = 0; s < splits; ++s) {
-                double2 x0[kI], x1[kI];
 #pragma unroll
-                for (int i = 0; i < kI; ++i) {
-                    const int o = tid + kEvdThreads * i, c = o >> 4, j = o & 15;
-                    const double *q = p + (size_t)s * 4096 + c * 64 + 4 * j;
-                    x0[i] = __ldg(reinterpret_cast<const double2 *>(q));
-                    x1[i] = __ldg(reinterpret_cast<const double2 *>(q + 2));
-                }
-#pragma unroll
-                for (int i = 0; i < kI; ++i) {
-                    acc[i][0] += x0[i].x;
-                    acc[i][1] += x0[i].y;
-                    acc[i][2] += x1[i].x;
-                    acc[i][3] += x1[i].y;
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kI; ++i) {
-            const int o = tid + kEvdThreads * i, c = o >> 4, j = o & 15;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int r = 4 * j + k;
-                if (kind == 0) {
-                    G1[r * kEvdTmpLD + c] = acc[i][k];
-                } else if (r <= c) {  // the FP64 Gram kernel writes the upper triangle only: mirror it
-                    G1[r * kEvdTmpLD + c] = acc[i][k];
-                    G1[c * kEvdTmpLD + r] = acc[i][k];
-                }
+            for (int h = 0; h < 2; ++h) {
+                const int rr = urow[i] + h;
+                if (rr > ucol[i]) continue;
+                G0[evd_off(evd_column_slot(rr), evd_column_slot(ucol[i]))] = acc[i][h];
+                if (rr == ucol[i]) dg[rr] = acc[i][h];
             }
         }
     }
-    // W: warp w < 8 holds rows 32 (w & 1) + lane, quarter w >> 1 of the slots
-    const int wrow = 32 * (warp & 1) + lane, quarter = (warp >> 1) & 3;
-    double w[16];
+    // W's identity: rows 32 (bulk & 1) + lane, quarter bulk >> 1
+    const int wrow = 32 * (bulk & 1) + lane, quarter = (bulk >> 1) & 3;
+    EvdRow w;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) w[j] = (evd_slot_column(16 * quarter + j) == wrow) ? 1.0 : 0.0;
+    for (int j = 0; j < 8; ++j) {
+        w.f[j] = 8 * quarter + j == wrow ? 1.0 : 0.0;
+        w.s[j] = 63 - 8 * quarter - j == wrow ? 1.0 : 0.0;
+    }
+    w.x0 = w.f[0];
+    w.y7 = w.s[7];
     __syncthreads();
-    // symmetrise (the two triangles come from different accumulation orders)
-    // into buffer 0 in slot coordinates, measure the input's largest scaled
-    // off-diagonal entry, and find whether any index pair passes the rotation
-    // test at all: if none does, no round can rotate (G never changes) and the
-    // solve is skipped
+    // the input's largest scaled off-diagonal entry, and whether any index pair
+    // passes the rotation test at all: if none does, no round can rotate (G
+    // never changes) and the solve is skipped
     double off = 0.0;
     int need = 0;
-    for (int e = tid; e < kW * kW; e += kEvdThreads) {
-        const int r = e >> 6, c = e & 63;
-        if (r <= c) {
-            const double g = r < c ? 0.5 * (G1[r * kEvdTmpLD + c] + G1[c * kEvdTmpLD + r]) : G1[r * kEvdTmpLD + r];
-            G0[evd_off(evd_column_slot(r), evd_column_slot(c))] = g;
-            if (r < c) {
-                const double a = fmax(G1[r * kEvdTmpLD + r], 0.0) * fmax(G1[c * kEvdTmpLD + c], 0.0);
-                const double d = sqrt(a);
-                if (d > 0.0) off = fmax(off, fabs(g) / d);
-                if (fabs(g) > 1.0e-300 && g * g > (tau * tau) * a) need = 1;
-            }
-        }
-    }
-    if (off > 0.0) atomicMax(&off_bits, (unsigned long long)__double_as_longlong(off));
-    // the off-diagonal 2 x 2 blocks a thread updates in every round: a group
-    // of 32 blocks per warp and iteration in which each half-warp holds every
-    // residue of a + b mod 16 once (shared memory serves a half-warp's 8-byte
-    // accesses per wavefront; groups 0-13: G warps 8-14, two each; group 14:
-    // warp 0; group 15, 16 blocks of odd residue: lanes 0-15 of warp 1).  Per block: the pair indices
-    // (a | b << 8), the offsets of FF[a][b] (FS[a][b] and SS[a][b] follow at
-    // fixed distances) and of FS[b][a], and the destinations of its four
-    // entries after the advance, two per int
-    int blk[kEvdBulkIters], rof[kEvdBulkIters], w01[kEvdBulkIters], w23[kEvdBulkIters];
 #pragma unroll
-    for (int j = 0; j < kEvdBulkIters; ++j) {
-        int g = -1;
-        if (warp >= 8 && warp < 15) g = 2 * (warp - 8) + j;
-        else if (j == 0 && warp == 0) g = 14;
-        else if (j == 0 && warp == 1 && lane < 16) g = 15;
-        blk[j] = -1;
-        rof[j] = w01[j] = w23[j] = 0;
-        if (g >= 0) {
-            const int2 ab = g < 15 ? evd_block_of(lane & 15, 2 * g + (lane >> 4))
-                                   : evd_block_of(2 * (lane & 7) + 1, 30 + (lane >> 3));
-            const int a = ab.x, b = ab.y;
-            const int pa = evd_next_slot(2 * a), qa = evd_next_slot(2 * a + 1);
-            const int pb = evd_next_slot(2 * b), qb = evd_next_slot(2 * b + 1);
-            blk[j] = a | (b << 8);
-            rof[j] = evd_off(2 * a, 2 * b) | (evd_off(2 * a + 1, 2 * b) << 16);
-            w01[j] = evd_off(pa, pb) | (evd_off(pa, qb) << 16);
-            w23[j] = evd_off(qa, pb) | (evd_off(qa, qb) << 16);
+    for (int i = 0; i < kI; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int rr = urow[i] + h;
+            if (rr >= ucol[i]) continue;
+            const double g = acc[i][h];
+            const double a = fmax(dg[rr], 0.0) * fmax(dg[ucol[i]], 0.0);
+            if (a > 0.0) off = fmax(off, fabs(g) * rsqrt(a));
+            if (fabs(g) > 1.0e-300 && g * g > (tau * tau) * a) need = 1;
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) off = fmax(off, __shfl_xor_sync(0xffffffffu, off, o));
+    if (lane == 0 && off > 0.0) atomicMax(&off_bits, (unsigned long long)__double_as_longlong(off));
+    // the blocks a G thread updates in every round (a lane without a second one
+    // reads the first entries and stores nothing)
+    EvdBlock blk[kEvdBulkIters] = {};
+    if (is_g) {
+#pragma unroll
+        for (int j = 0; j < kEvdBulkIters; ++j) {
+            const int4 v = __ldg(
+                reinterpret_cast<const int4 *>(&kEvdBlocks.of[kEvdBulkIters * (bulk - kEvdW) + j][lane]));
+            blk[j] = EvdBlock{v.x, v.y, v.z, v.w};
         }
     }
-    const bool work = __syncthreads_or(need) != 0;
-    // warp 15, lane k = pair k: its diagonal block's destinations, the block
-    // (A, B) holding the off-diagonal entry of its next pair, and its state
-    // from round to round: the pair's entries and rotation (pp, qq, pq, c, s,
-    // t, rotated), the rotated diagonals nd0, nd1, the next pair's diagonal
-    // part of the rotation (pre) and the angles of pairs A and B
-    const int A = lane <= 1 ? 0 : lane - 1, RA = lane == 1 ? 1 : 0;
-    const int B = lane <= 30 ? lane + 1 : 31, RB = lane <= 30 ? 1 : 0;
-    const int dpp = evd_off(evd_next_slot(2 * lane), evd_next_slot(2 * lane));
-    const int dqq = evd_off(evd_next_slot(2 * lane + 1), evd_next_slot(2 * lane + 1));
-    const int dpq = evd_off(evd_next_slot(2 * lane), evd_next_slot(2 * lane + 1));
-    const int rab = evd_off(2 * A, 2 * B), rba = evd_off(2 * A + 1, 2 * B);
-    double a_pq = 0.0, a_c = 1.0, a_s = 0.0, a_t = 0.0, nd0 = 0.0, nd1 = 0.0, ca = 1.0, sa = 0.0, cb = 1.0, sb = 0.0;
-    double n_pp = 0.0, n_qq = 0.0;
-    bool me = false;
-    EvdPre pre{0.0, 0.0, 0.0};
-    // after the angles of a round are known: the rotated diagonals, the next
-    // pair's diagonal entries and diagonal part, and the angles of A and B
-    auto prepare_next = [&](double pp, double qq) {
-        nd0 = fma(-a_t, a_pq, pp);
-        nd1 = fma(a_t, a_pq, qq);
-        // first index of pair k: pair k-1's first (k >= 2), pair 0's second
-        // (k = 1), its own (k = 0); second index: pair k+1's second (k <= 30),
-        // its own first (k = 31)
-        const double up = __shfl_up_sync(0xffffffffu, lane == 0 ? nd1 : nd0, 1);
-        const double dn = __shfl_down_sync(0xffffffffu, nd1, 1);
-        ca = __shfl_sync(0xffffffffu, a_c, A);
-        sa = __shfl_sync(0xffffffffu, a_s, A);
-        cb = __shfl_sync(0xffffffffu, a_c, B);
-        sb = __shfl_sync(0xffffffffu, a_s, B);
-        n_pp = lane == 0 ? nd0 : up;
-        n_qq = lane == 31 ? nd0 : dn;
-        pre = evd_prepare(n_pp, n_qq, tau);
-    };
-    if (warp == 15 && work) {
-        const double pp = G0[evd_off(2 * lane, 2 * lane)];
-        const double qq = G0[evd_off(2 * lane + 1, 2 * lane + 1)];
-        a_pq = G0[evd_off(2 * lane, 2 * lane + 1)];
-        me = evd_rotation(evd_prepare(pp, qq, tau), a_pq, a_c, a_s, a_t);
-        cs[0][lane] = make_double2(a_c, a_s);
-        cs_c[0][lane] = a_c;
-        cs_s[0][lane] = a_s;
-        const unsigned m = __ballot_sync(0xffffffffu, me);
-        if (lane == 0) {
-            rot_mask[0] = m;
-            if (m) sweep_any[0] = 1;
-        }
-        prepare_next(pp, qq);
-    }
+    const bool second = bulk < kEvdBulk - 1 || lane < 16;  // this lane has a second block
+    const bool work = __syncthreads_or(need) != 0 && nsweeps > 0;
     bool rotated_any = false;
     int gr = 0;  // rounds executed so far (buffer parity)
-    for (int sw = 0; sw < (work ? nsweeps : 0); ++sw) {
-        for (int r = 0; r < kEvdRounds; ++r, ++gr) {
-            __syncthreads();  // round gr's angles published, its input buffer complete
+    // Round bookkeeping common to the roles: after round gr's work, whether
+    // another round follows.  sweep_any[sw] was last written before the final
+    // barrier of sweep sw.
+    int r = 0, sw = 0;
+    auto next_round = [&]() -> bool {
+        ++gr;
+        if (++r < kEvdRounds) return true;
+        r = 0;
+        if (!sweep_any[sw]) return false;  // the same value in every thread
+        rotated_any = true;
+        return ++sw < nsweeps;
+    };
+    constexpr int kRoundBar = 1;
+    if (work && is_angle) {
+        // lane k = pair k: its diagonal block's destinations, the block (A, B)
+        // holding the off-diagonal entry of its next pair, and its state from
+        // round to round: the pair's entries and rotation (pq, c, s, t,
+        // rotated), the rotated diagonals nd0, nd1, the next pair's diagonal
+        // part of the rotation (pre) and the angles of pairs A and B
+        const int A = lane <= 1 ? 0 : lane - 1, RA = lane == 1 ? 1 : 0;
+        const int B = lane <= 30 ? lane + 1 : 31, RB = lane <= 30 ? 1 : 0;
+        const int dpp = evd_off(evd_next_slot(2 * lane), evd_next_slot(2 * lane));
+        const int dqq = evd_off(evd_next_slot(2 * lane + 1), evd_next_slot(2 * lane + 1));
+        const int dpq = evd_off(evd_next_slot(2 * lane), evd_next_slot(2 * lane + 1));
+        const int rab = evd_off(2 * A, 2 * B), rba = evd_off(2 * A + 1, 2 * B);
+        const double tau2 = tau * tau;
+        double a_pq, a_c, a_s, a_t, nd0, nd1, n_pp, n_qq;
+        bool me;
+        // after the angles of a round are known: the rotated diagonals and the
+        // next pair's diagonal entries
+        auto prepare_next = [&](double pp, double qq) {
+            nd0 = fma(-a_t, a_pq, pp);
+            nd1 = fma(a_t, a_pq, qq);
+            // first index of pair k: pair k-1's first (k >= 2), pair 0's second
+            // (k = 1), its own (k = 0); second index: pair k+1's second (k <= 30),
+            // its own first (k = 31)
+            const double up = __shfl_up_sync(0xffffffffu, lane == 0 ? nd1 : nd0, 1);
+            const double dn = __shfl_down_sync(0xffffffffu, nd1, 1);
+            n_pp = lane == 0 ? nd0 : up;
+            n_qq = lane == 31 ? nd0 : dn;
+        };
+        auto publish = [&](int parity, int sweep) {
+            cs[parity][lane] = make_double2(a_c, a_s);
+            cs_c[parity][lane] = a_c;
+            cs_s[parity][lane] = a_s;
+            if (me) sweep_any[sweep] = 1;
+        };
+        n_pp = G0[evd_off(2 * lane, 2 * lane)];
+        n_qq = G0[evd_off(2 * lane + 1, 2 * lane + 1)];
+        a_pq = G0[evd_off(2 * lane, 2 * lane + 1)];
+        me = evd_rotation(n_pp, n_qq, tau2, a_pq, a_c, a_s, a_t);
+        publish(0, 0);
+        prepare_next(n_pp, n_qq);
+        do {
+            group_barrier(kRoundBar, kEvdLoopThreads);  // round gr's angles published, its input buffer complete
             const int cur = gr & 1;
             const double *Gin = cur ? G1 : G0;
             double *Gout = cur ? G0 : G1;
-            if (warp < 8) {
-                if (gr > 0) {  // the advance after round gr - 1 (its boundary values are published)
-                    const int pb = gr & 1;
-                    const double up = quarter > 0 ? xf[pb][quarter - 1][wrow] : 0.0;
-                    const double down = quarter < 3 ? xs[pb][quarter + 1][wrow] : 0.0;
-                    evd_w_advance(w, quarter, up, down);
-                }
-                if (rot_mask[cur]) evd_w_rotate(w, cs[cur], quarter);
-                xf[cur ^ 1][quarter][wrow] = w[14];
-                xs[cur ^ 1][quarter][wrow] = w[1];
-            }
-            if (warp < 15) {
+            // block (A, B), A < B: FF[A][B], FS[A][B], FS[B][A], SS[A][B], and
+            // the angles of pairs A and B
+            const double g11 = Gin[rab], g12 = Gin[rab + kEvdQuad], g22 = Gin[rab + 2 * kEvdQuad];
+            const double g21 = Gin[rba];
+            const double2 ra = cs[cur][A], rb = cs[cur][B];
+            // element (RA, RB) of block (A, B) of this round's output, as the
+            // update computes it: h_i = ux g_i1 + uy g_i2, then vx h_1 + vy h_2
+            const double ux = RB ? rb.y : rb.x, uy = RB ? rb.x : -rb.y;
+            const double vx = RA ? ra.y : ra.x, vy = RA ? ra.x : -ra.y;
+            const double h1 = fma(ux, g11, uy * g12), h2 = fma(ux, g21, uy * g22);
+            const double old_pq = a_pq;
+            a_pq = fma(vx, h1, vy * h2);
+            // round gr's diagonal block of pair k: g_pp - t g_pq, g_qq + t g_pq, 0
+            Gout[dpp] = nd0;
+            Gout[dqq] = nd1;
+            Gout[dpq] = me ? 0.0 : old_pq;
+            me = evd_rotation(n_pp, n_qq, tau2, a_pq, a_c, a_s, a_t);
+            publish(cur ^ 1, r + 1 < kEvdRounds ? sw : sw + 1);
+            prepare_next(n_pp, n_qq);
+        } while (next_round());
+        if (lane == 0) s_rounds = gr;
+    } else if (work && is_g) {
+        do {
+            group_barrier(kRoundBar, kEvdLoopThreads);
+            const int cur = gr & 1;
+            const double *Gin = cur ? G1 : G0;
+            double *Gout = cur ? G0 : G1;
+            // both blocks' loads first: a load cannot pass a store to G
+            double2 P[kEvdBulkIters], Q[kEvdBulkIters];
+            double g11[kEvdBulkIters], g12[kEvdBulkIters], g21[kEvdBulkIters], g22[kEvdBulkIters];
 #pragma unroll
-                for (int j = 0; j < kEvdBulkIters; ++j) {
-                    if (blk[j] < 0) continue;
-                    const int ia = blk[j] & 255, ib = blk[j] >> 8;
-                    const double2 P = make_double2(cs_c[cur][ia], cs_s[cur][ia]);
-                    const double2 Q = make_double2(cs_c[cur][ib], cs_s[cur][ib]);
-                    const double *f = Gin + (rof[j] & 0xffff);
-                    const double g11 = f[0], g12 = f[kEvdQuad], g22 = f[2 * kEvdQuad], g21 = Gin[rof[j] >> 16];
-                    // columns: [p' q'] = [c p - s q, s p + c q] (on the right, pair b)
-                    const double h11 = fma(Q.x, g11, -(Q.y * g12)), h12 = fma(Q.y, g11, Q.x * g12);
-                    const double h21 = fma(Q.x, g21, -(Q.y * g22)), h22 = fma(Q.y, g21, Q.x * g22);
-                    // rows (on the left, pair a)
-                    Gout[w01[j] & 0xffff] = fma(P.x, h11, -(P.y * h21));
-                    Gout[w01[j] >> 16] = fma(P.x, h12, -(P.y * h22));
-                    Gout[w23[j] & 0xffff] = fma(P.y, h11, P.x * h21);
-                    Gout[w23[j] >> 16] = fma(P.y, h12, P.x * h22);
-                }
-            } else {
-                // block (A, B), A < B: FF[A][B], FS[A][B], FS[B][A], SS[A][B]
-                const double g11 = Gin[rab], g12 = Gin[rab + kEvdQuad], g22 = Gin[rab + 2 * kEvdQuad];
-                const double g21 = Gin[rba];
-                // round gr's diagonal block of pair k: g_pp - t g_pq, g_qq + t g_pq, 0
-                Gout[dpp] = nd0;
-                Gout[dqq] = nd1;
-                Gout[dpq] = me ? 0.0 : a_pq;
-                // element (RA, RB) of block (A, B) of G_out, as the update computes it
-                const double h1 = RB ? fma(sb, g11, cb * g12) : fma(cb, g11, -(sb * g12));  // h1RB
-                const double h2 = RB ? fma(sb, g21, cb * g22) : fma(cb, g21, -(sb * g22));  // h2RB
-                a_pq = RA ? fma(sa, h1, ca * h2) : fma(ca, h1, -(sa * h2));
-                me = evd_rotation(pre, a_pq, a_c, a_s, a_t);
-                cs[cur ^ 1][lane] = make_double2(a_c, a_s);
-                cs_c[cur ^ 1][lane] = a_c;
-                cs_s[cur ^ 1][lane] = a_s;
-                const unsigned m = __ballot_sync(0xffffffffu, me);
-                if (lane == 0) {
-                    rot_mask[cur ^ 1] = m;
-                    if (m) sweep_any[r + 1 < kEvdRounds ? sw : sw + 1] = 1;
-                }
-                prepare_next(n_pp, n_qq);
+            for (int j = 0; j < kEvdBulkIters; ++j) {
+                const int ia = blk[j].ab & 255, ib = blk[j].ab >> 8;
+                const double *f = Gin + (blk[j].rof & 0xffff);
+                Q[j] = make_double2(cs_c[cur][ib], cs_s[cur][ib]);
+                g11[j] = f[0];
+                g12[j] = f[kEvdQuad];
+                g22[j] = f[2 * kEvdQuad];
+                g21[j] = Gin[blk[j].rof >> 16];
+                P[j] = make_double2(cs_c[cur][ia], cs_s[cur][ia]);
             }
+#pragma unroll
+            for (int j = 0; j < kEvdBulkIters; ++j) {
+                // columns: [p' q'] = [c p - s q, s p + c q] (on the right, pair b)
+                const double h11 = fma(Q[j].x, g11[j], -(Q[j].y * g12[j])), h12 = fma(Q[j].y, g11[j], Q[j].x * g12[j]);
+                const double h21 = fma(Q[j].x, g21[j], -(Q[j].y * g22[j])), h22 = fma(Q[j].y, g21[j], Q[j].x * g22[j]);
+                // rows (on the left, pair a)
+                g11[j] = fma(P[j].x, h11, -(P[j].y * h21));
+                g12[j] = fma(P[j].x, h12, -(P[j].y * h22));
+                g21[j] = fma(P[j].y, h11, P[j].x * h21);
+                g22[j] = fma(P[j].y, h12, P[j].x * h22);
+            }
+#pragma unroll
+            for (int j = 0; j < kEvdBulkIters; ++j) {
+                if (j == 0 || second) {
+                    Gout[blk[j].w01 & 0xffff] = g11[j];
+                    Gout[blk[j].w01 >> 16] = g12[j];
+                    Gout[blk[j].w23 & 0xffff] = g21[j];
+                    Gout[blk[j].w23 >> 16] = g22[j];
+                }
+            }
+        } while (next_round());
+    } else if (work && is_w) {
+        auto round = [&](auto phase) -> bool {
+            constexpr int ph = decltype(phase)::value;
+            group_barrier(kRoundBar, kEvdLoopThreads);
+            const int cur = gr & 1;
+            if (gr > 0) {  // what the neighbouring quarters published in round gr - 1
+                if (quarter > 0) w.x0 = xf[cur][quarter - 1][wrow];
+                if (quarter < 3) w.y7 = xs[cur][quarter + 1][wrow];
+            }
+            double lf, fs;
+            evd_w_round<ph>(w, cs[cur], quarter, lf, fs);
+            xf[cur ^ 1][quarter][wrow] = lf;
+            xs[cur ^ 1][quarter][wrow] = fs;
+            if (quarter == 3) w.y7 = lf;
+            return next_round();
+        };
+        for (;;) {
+            if (!round(std::integral_constant<int, 0>{})) break;
+            if (!round(std::integral_constant<int, 1>{})) break;
+            if (!round(std::integral_constant<int, 2>{})) break;
+            if (!round(std::integral_constant<int, 3>{})) break;
+            if (!round(std::integral_constant<int, 4>{})) break;
+            if (!round(std::integral_constant<int, 5>{})) break;
+            if (!round(std::integral_constant<int, 6>{})) break;
+            if (!round(std::integral_constant<int, 7>{})) break;
         }
-        // sweep_any[sw] was last written before this sweep's final barrier
-        if (!sweep_any[sw]) break;  // the same value in every thread
-        rotated_any = true;
     }
-    __syncthreads();  // the last round's output buffer and W boundary values are complete
-    if (warp < 8 && gr > 0) {  // the advance after the last round
+    // the last round's output buffer and W boundary values are complete; every
+    // thread learns whether something rotated
+    rotated_any = __syncthreads_or(rotated_any) != 0;
+    if (work && is_w) {  // the advance after the last round
         const int pb = gr & 1;
-        const double up = quarter > 0 ? xf[pb][quarter - 1][wrow] : 0.0;
-        const double down = quarter < 3 ? xs[pb][quarter + 1][wrow] : 0.0;
-        evd_w_advance(w, quarter, up, down);
+        if (quarter > 0) w.x0 = xf[pb][quarter - 1][wrow];
+        if (quarter < 3) w.y7 = xs[pb][quarter + 1][wrow];
     }
-    const double *Gf = (gr & 1) ? G1 : G0;
+    const double *Gf = (s_rounds & 1) ? G1 : G0;
     // Output order of W's columns.  With `sort`, the eigenvalues (G's
     // diagonal) are ranked and the lower-numbered block of the pair receives
     // the larger ones (decreasing norms across the blocks, de Rijk's
@@ -994,7 +991,7 @@ __global__ void __launch_bounds__(kEvdThreads, 1)
     // (global index < ncols) are reordered, among their own positions: the
     // zero padding columns never rotate and must stay at the end.  After full
     // sweeps the slots are back at their starting columns.
-    if (rotated_any) {  // the same value in every thread
+    if (rotated_any && tid < 8 * kW) {  // the same value in every thread of a warp
         // column col = tid / 8 is compared with columns 8 part .. 8 part + 7
         // (part = tid % 8) and the 8 counts meet over lanes xor 1, 2, 4
         const int col = tid >> 3, part = tid & 7;
@@ -1026,14 +1023,27 @@ __global__ void __launch_bounds__(kEvdThreads, 1)
         }
     }
     __syncthreads();
-    if (rotated_any && tid < kEvdWThreads) {
-        // every sweep ran all 63 rounds: slot s holds column evd_slot_column(s)
-        double *wo = Wout + (size_t)pair * kW * kW;
+    if (rotated_any) {
+        if (is_w) {
+            // every sweep ran all 63 rounds: slot s holds column evd_slot_column(s)
+            auto store = [&](int slot, double v) { Ws[out_col[evd_slot_column(slot)] * kEvdWLD + wrow] = v; };
+            const int ph = gr & 7;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int col = out_col[evd_slot_column(16 * quarter + j)];
-            wo[(size_t)col * kW + wrow] = w[j];
-            if (Wimg != nullptr) rot_b_store(Wimg + (size_t)pair * kRotImgFloats, wrow, col, w[j]);
+            for (int i = 0; i < 8; ++i) {
+                const int jf = (i + ph) & 7, js = (i - ph) & 7;  // the logical pairs of these registers
+                store(16 * quarter + 2 * jf, jf == 0 ? w.x0 : w.f[i]);
+                store(16 * quarter + 2 * js + 1, js == 7 ? w.y7 : w.s[i]);
+            }
+        }
+        __syncthreads();
+        double *wo = Wout + (size_t)pair * kW * kW;
+        float *img = Wimg + (size_t)pair * kRotImgFloats;
+        const int row = tid & (kW - 1);
+#pragma unroll 6
+        for (int col = tid >> 6; col < kW; col += kEvdThreads / kW) {
+            const double v = Ws[col * kEvdWLD + row];
+            wo[col * kW + row] = v;
+            if (Wimg != nullptr) rot_b_store(img, row, col, v);
         }
     }
     if (tid == 0) {
@@ -1158,27 +1168,17 @@ __global__ void mx_half_step(double *__restrict__ E, int n)
         E[e] = ((e / n == e % n) ? 1.0 : 0.0) - 0.5 * E[e];
 }
 
-// g[pair] (64 x 64 column-major FP64) = sum of the pair's Gram partials
-__global__ void mx_sum_partials(const void *__restrict__ part, int kind, int splits, int npairs, double *__restrict__ g)
+// g[pair] (64 x 64 column-major FP64, both triangles) = sum of the pair's Gram
+// partials (upper triangles)
+__global__ void mx_sum_partials(const double *__restrict__ part, int splits, int npairs, double *__restrict__ g)
 {
     const size_t total = (size_t)npairs * kW * kW;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const int pair = (int)(e / (kW * kW)), rc = (int)(e % (kW * kW));
-        int r = rc & 63, c = rc >> 6;
-        if (kind != 0 && r > c) {  // the FP64 Gram holds the upper triangle: read the mirror
-            const int t = r;
-            r = c;
-            c = t;
-        }
+        const int r = min(rc & 63, rc >> 6), c = max(rc & 63, rc >> 6);
+        const double *p = part + (size_t)pair * splits * 4096;
         double acc = 0.0;
-        if (kind == 0) {
-            const float *p = static_cast<const float *>(part) + (size_t)pair * splits * 8192;
-            for (int s = 0; s < splits; ++s)
-                acc += (double)p[(size_t)s * 8192 + c * 128 + r] + (double)p[(size_t)s * 8192 + c * 128 + r + 64];
-        } else {
-            const double *p = static_cast<const double *>(part) + (size_t)pair * splits * 4096;
-            for (int s = 0; s < splits; ++s) acc += p[(size_t)s * 4096 + c * 64 + r];
-        }
+        for (int s = 0; s < splits; ++s) acc += p[(size_t)s * 4096 + c * 64 + r];
         g[e] = acc;
     }
 }
@@ -1448,13 +1448,13 @@ int run_sweep(Work &w, bool tc, double tau, int inner, int sort, cudaStream_t st
         if (si >= 0) cudaEventRecord(w.tev[si][0], st);
         if (tc) {
             mx_gram_tc<<<dim3(w.tc_splits, w.npairs), kGramTcThreads, kGramTcSmem, st>>>(
-                w.mxh, w.mxl, w.nb, r, w.tc_chunks, w.tc_chunks_per_split, static_cast<float *>(w.part), w.status);
+                w.mxh, w.mxl, w.nb, r, w.tc_chunks, w.tc_chunks_per_split, static_cast<double *>(w.part), w.status);
             if (si >= 0) {
                 cudaEventRecord(w.tev[si][1], st);
                 cudaMemcpyAsync(w.stats + 4 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
             }
-            mx_evd<<<w.npairs, kEvdThreads, kEvdSmem, st>>>(w.part, 0, w.tc_splits, tau, inner, w.nb, r, sort, w.cols,
-                                                            w.W, w.wimg, w.flags, w.stats);
+            mx_evd<<<w.npairs, kEvdThreads, kEvdSmem, st>>>(static_cast<const double *>(w.part), w.tc_splits, tau, inner,
+                                                            w.nb, r, sort, w.cols, w.W, w.wimg, w.flags, w.stats);
             if (si >= 0) {
                 cudaMemcpyAsync(w.stats + 5 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
                 cudaEventRecord(w.tev[si][2], st);
@@ -1471,8 +1471,8 @@ int run_sweep(Work &w, bool tc, double tau, int inner, int sort, cudaStream_t st
                 cudaEventRecord(w.tev[si][1], st);
                 cudaMemcpyAsync(w.stats + 4 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
             }
-            mx_evd<<<w.npairs, kEvdThreads, kEvdSmem, st>>>(w.part, 1, w.f64_splits, tau, inner, w.nb, r, sort,
-                                                            w.cols, w.W, nullptr, w.flags, w.stats);
+            mx_evd<<<w.npairs, kEvdThreads, kEvdSmem, st>>>(static_cast<const double *>(w.part), w.f64_splits, tau, inner,
+                                                            w.nb, r, sort, w.cols, w.W, nullptr, w.flags, w.stats);
             if (si >= 0) {
                 cudaMemcpyAsync(w.stats + 5 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
                 cudaEventRecord(w.tev[si][2], st);
@@ -1813,13 +1813,14 @@ extern "C" int jsvd_mixed_test_round(int kind, double *d_x, int rows, int cols, 
         if (tc) mx_split<<<grid_for(mn), 256, 0, st>>>(d_x, mn, w.xh, w.xl);
         if (kind == 0) {
             mx_gram_tc<<<dim3(w.tc_splits, w.npairs), kGramTcThreads, kGramTcSmem, st>>>(
-                w.mxh, w.mxl, w.nb, round, w.tc_chunks, w.tc_chunks_per_split, static_cast<float *>(w.part), w.status);
-            mx_sum_partials<<<grid_for((size_t)w.npairs * 4096), 256, 0, st>>>(w.part, 0, w.tc_splits, w.npairs, d_gw);
+                w.mxh, w.mxl, w.nb, round, w.tc_chunks, w.tc_chunks_per_split, static_cast<double *>(w.part), w.status);
+            mx_sum_partials<<<grid_for((size_t)w.npairs * 4096), 256, 0, st>>>(
+                static_cast<const double *>(w.part), w.tc_splits, w.npairs, d_gw);
         } else if (kind == 1) {
             mx_gram_f64<<<dim3(w.f64_splits, w.npairs), kGram64Threads, kGram64Smem, st>>>(
                 d_x, rows, w.nb, round, w.f64_rows_per_split, rows, static_cast<double *>(w.part));
-            mx_sum_partials<<<grid_for((size_t)w.npairs * 4096), 256, 0, st>>>(w.part, 1, w.f64_splits, w.npairs,
-                                                                                d_gw);
+            mx_sum_partials<<<grid_for((size_t)w.npairs * 4096), 256, 0, st>>>(
+                static_cast<const double *>(w.part), w.f64_splits, w.npairs, d_gw);
         } else {
             mx_fill_int<<<1, 256, 0, st>>>(w.flags, w.npairs, 1);
             if (kind == 2) {

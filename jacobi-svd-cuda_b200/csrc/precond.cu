@@ -111,10 +111,8 @@ __global__ void __launch_bounds__(256) pc_shift_diagonal(double *__restrict__ G,
 // status <- 1 on a pivot that is not positive and finite.
 constexpr int kDiagThreads = 384;
 
-// 1 / d for a pivot d: from the hardware's approximation r (relative error
-// e = 1 - d r of about 2^-20) as r (1 + e + e^2).  A pivot outside the
-// approximation's range is divided by; one that is not positive and finite is
-// replaced by 1 and clears ok.
+// 1 / d for a pivot d.  A pivot outside the approximation's range is divided
+// by; one that is not positive and finite is replaced by 1 and clears ok.
 __device__ __noinline__ double pc_reciprocal_rare(double &d, bool &ok)
 {
     if (!(d > 0.0 && d < INFINITY)) {
@@ -126,12 +124,8 @@ __device__ __noinline__ double pc_reciprocal_rare(double &d, bool &ok)
 
 __device__ __forceinline__ double pc_reciprocal(double &d, bool &ok)
 {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double e = fma(-d, r, 1.0);
-    r = fma(r, fma(e, e, e), r);
-    const unsigned hi = (unsigned)__double2hiint(d);  // 2^-1000 <= d < 2^1000
-    if (hi - 0x01700000u >= 0x7e700000u - 0x01700000u) r = pc_reciprocal_rare(d, ok);
+    double r = approx_reciprocal(d);
+    if (!reciprocal_in_range(d)) r = pc_reciprocal_rare(d, ok);
     return r;
 }
 
