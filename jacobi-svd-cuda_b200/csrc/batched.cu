@@ -9,10 +9,10 @@
 //   class 3  : A in shared memory, V in a per-CTA slice of global memory
 //   class 4  : A and V in global memory (L2-resident per-CTA slices), the
 //              leading columns of A that fit in shared memory kept there
-// By default the members of classes 3 and 4 are instead solved by a
-// thread-block cluster each (batch_cluster_kernel: A and V in the cluster's
-// distributed shared memory; see the section "cluster classes"); a member no
-// cluster holds stays with its class's kernel.
+// By default the members of class 4 are instead solved by a thread-block
+// cluster each (batch_cluster_kernel: A and V in the cluster's distributed
+// shared memory; see the section "cluster classes"); a member no cluster holds
+// stays with its class's kernel.
 // Launch shapes per class (threads, CTAs per SM, grid cap) come from the
 // compiled-in table batch_tuning_table.h, which batch_autotune.py writes from
 // jsvd_batch_autotune (defined at the end of this file).
@@ -47,29 +47,75 @@ constexpr int kLanes = 256;      // reduction width T (reference default)
 constexpr int kW = kLanes / 32;  // virtual lanes per physical lane
 constexpr int kClasses = 5;
 
-// Reference-order dot products of columns x, y (length m) by one warp; the
-// totals are valid in lane 0.
-__device__ __forceinline__ void warp_pair_stats(const double *x, const double *y, int m, int lane, double &pp,
-                                                double &qq, double &pq)
+// The in-warp levels 16 .. 1 of the reference's tree for the three sums of a
+// pair at once: at each level a lane keeps one of two quantities and hands the
+// other over (the operands of an addition commute, so each total meets in the
+// reference's order).  Six exchanges instead of fifteen.  The totals end up in
+// lane 0 (pp), lane 8 (pq) and lane 16 (qq); every lane returns the one of its
+// lane / 8.
+__device__ __forceinline__ double warp_tree3(double pp, double qq, double pq, int lane)
 {
-    double app[kW], aqq[kW], apq[kW];
+    const bool hi = (lane & 16) != 0;
+    const double give = hi ? pp : qq;
+    double a = hi ? qq : pp;  // pp below lane 16, qq from there
+    a += __shfl_xor_sync(0xffffffffu, give, 16);
+    pq += __shfl_xor_sync(0xffffffffu, pq, 16);
+    const bool mid = (lane & 8) != 0;
+    const double give2 = mid ? a : pq;
+    double b = mid ? pq : a;
+    b += __shfl_xor_sync(0xffffffffu, give2, 8);
+    b += __shfl_xor_sync(0xffffffffu, b, 4);
+    b += __shfl_xor_sync(0xffffffffu, b, 2);
+    b += __shfl_xor_sync(0xffffffffu, b, 1);
+    return b;
+}
+
+// Reference-order dot products of columns x, y (length m) by one warp, as
+// warp_tree3 returns them.  NJ > 0: at most 32 NJ rows (NJ <= kW), one per
+// virtual lane and none beyond; NJ = 0: any number.  A virtual lane's single
+// product is its sum (fma with a zero rounds it the same way).
+template <int NJ>
+__device__ __forceinline__ double warp_pair_stats(const double *x, const double *y, int m, int lane)
+{
+    constexpr int J = NJ > 0 ? NJ : kW;
+    double app[J], aqq[J], apq[J];
+    if constexpr (NJ > 0) {
 #pragma unroll
-    for (int j = 0; j < kW; ++j) app[j] = aqq[j] = apq[j] = 0.0;
-    for (int base = 0; base < m; base += kLanes) {
-#pragma unroll
-        for (int j = 0; j < kW; ++j) {
-            const int r = base + 32 * j + lane;
+        for (int j = 0; j < J; ++j) {
+            const int r = 32 * j + lane;
+            app[j] = aqq[j] = apq[j] = 0.0;
             if (r < m) {
                 const double a = x[r], b = y[r];
-                app[j] = fma(a, a, app[j]);
-                aqq[j] = fma(b, b, aqq[j]);
-                apq[j] = fma(a, b, apq[j]);
+                app[j] = a * a;
+                aqq[j] = b * b;
+                apq[j] = a * b;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < J; ++j) app[j] = aqq[j] = apq[j] = 0.0;
+        for (int base = 0; base < m; base += kLanes) {
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const int r = base + 32 * j + lane;
+                if (r < m) {
+                    const double a = x[r], b = y[r];
+                    app[j] = fma(a, a, app[j]);
+                    aqq[j] = fma(b, b, aqq[j]);
+                    apq[j] = fma(a, b, apq[j]);
+                }
             }
         }
     }
-    pp = warp_tree<kW>(app);
-    qq = warp_tree<kW>(aqq);
-    pq = warp_tree<kW>(apq);
+#pragma unroll
+    for (int s = J / 2; s >= 1; s >>= 1)
+#pragma unroll
+        for (int w = 0; w < s; ++w) {
+            app[w] += app[w + s];
+            aqq[w] += aqq[w + s];
+            apq[w] += apq[w + s];
+        }
+    return warp_tree3(app[0], aqq[0], apq[0], lane);
 }
 
 // Rotation of one column pair of A (length m) and of V (length n) by one
@@ -77,14 +123,46 @@ __device__ __forceinline__ void warp_pair_stats(const double *x, const double *y
 // before any store: with the working copies in global memory a load -> rotate
 // -> store loop pays one L2 round trip per 32 rows, because the compiler cannot
 // move a load past a store to a possibly aliasing column.
+// NJ > 0: m and n are at most 32 NJ; NJ = 0: any length.  kApart (everything in
+// shared memory, where the round trip is short): A's columns first, then V's,
+// in half the registers.
+template <int J>
+__device__ __forceinline__ void warp_rotate_columns(double *x, double *y, int m, int lane, double c, double s)
+{
+    double xa[J], ya[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const int r = 32 * j + lane;
+        if (r < m) {
+            xa[j] = x[r];
+            ya[j] = y[r];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const int r = 32 * j + lane;
+        if (r < m) {
+            x[r] = rot_p(c, s, xa[j], ya[j]);
+            y[r] = rot_q(c, s, xa[j], ya[j]);
+        }
+    }
+}
+
+template <int NJ, bool kApart>
 __device__ __forceinline__ void warp_rotate(double *x, double *y, int m, double *vx, double *vy, int n, int lane,
                                             double c, double s)
 {
-    const int len = m > n ? m : n;
+    if constexpr (NJ > 0 && kApart) {
+        warp_rotate_columns<NJ>(x, y, m, lane, c, s);
+        warp_rotate_columns<NJ>(vx, vy, n, lane, c, s);
+        return;
+    }
+    constexpr int J = NJ > 0 ? NJ : kW;
+    const int len = NJ > 0 ? 1 : (m > n ? m : n);
     for (int base = 0; base < len; base += kLanes) {
-        double xa[kW], ya[kW], xv[kW], yv[kW];
+        double xa[J], ya[J], xv[J], yv[J];
 #pragma unroll
-        for (int j = 0; j < kW; ++j) {
+        for (int j = 0; j < J; ++j) {
             const int r = base + 32 * j + lane;
             if (r < m) {
                 xa[j] = x[r];
@@ -96,7 +174,7 @@ __device__ __forceinline__ void warp_rotate(double *x, double *y, int m, double 
             }
         }
 #pragma unroll
-        for (int j = 0; j < kW; ++j) {
+        for (int j = 0; j < J; ++j) {
             const int r = base + 32 * j + lane;
             if (r < m) {
                 x[r] = rot_p(c, s, xa[j], ya[j]);
@@ -131,29 +209,29 @@ __host__ __device__ constexpr int round_half(int n) { return (n / 2 + 2) & ~1; }
 __host__ __device__ constexpr size_t round_scratch_doubles(int n) { return (size_t)5 * round_half(n); }
 
 // One sweep (every round of the circle) of an m x n member whose columns
-// colA(c) and V live wherever the caller keeps them, by the whole CTA; true
-// when some pair rotated.  s_rot must be 0 on entry and is 0 again on return.
-// The same phases and operations as one sweep of batch_kernel (which keeps
-// its own copy of the loop: sharing it raised that kernel's register spills).
-template <class ColA>
-__device__ __forceinline__ bool batch_sweep(ColA colA, double *V, int m, int n, double eps, double *st_pp,
-                                            double *st_qq, double *st_pq, double2 *st_cs, int &s_rot)
+// colA(c) and V live wherever the caller keeps them, by the whole CTA.  NJ as
+// in warp_pair_stats, for members of at most 32 NJ rows.  With one pair of
+// loops for any number of rows a 40-row member spent most of its instructions
+// on rows that it does not have, and with the loops for every bound in one
+// kernel the longest ones spilled; a kernel per bound, divisions out of the
+// schedule and six exchanges per tree instead of fifteen: 3000 FP64 members of
+// 16..64 rows 18.0 -> 5.8 ms, class 2 (397 members of up to 226 KiB) 24.6 ->
+// 17.6, 100 members of 228 x 189 with V in global memory 48 -> 31 (B200).
+template <int NJ, bool kApart, class ColA>
+__device__ __forceinline__ void sweep_rounds(ColA colA, double *V, int m, int n, double eps, double *st_pp,
+                                             double *st_qq, double *st_pq, double2 *st_cs, int &s_rot)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int ne = n + (n & 1);
     const int rounds = n >= 2 ? ne - 1 : 0;
     const int npairs = n / 2;
+    double *const st_mine = lane == 0 ? st_pp : (lane == 8 ? st_pq : st_qq);  // the total this lane holds
     for (int r = 0; r < rounds; ++r) {
         // phase 1: dot products, one warp per pair
         for (int k = warp; k < npairs; k += nwarps) {
             const int2 pq = round_robin_pair(n, r, k);
-            double pp, qq, pqv;
-            warp_pair_stats(colA(pq.x), colA(pq.y), m, lane, pp, qq, pqv);
-            if (lane == 0) {
-                st_pp[k] = pp;
-                st_qq[k] = qq;
-                st_pq[k] = pqv;
-            }
+            const double total = warp_pair_stats<NJ>(colA(pq.x), colA(pq.y), m, lane);
+            if (lane == 0 || lane == 8 || lane == 16) st_mine[k] = total;
         }
         __syncthreads();
         // phase 2: angles, one thread per pair
@@ -168,9 +246,41 @@ __device__ __forceinline__ bool batch_sweep(ColA colA, double *V, int m, int n, 
             const double2 g = st_cs[k];
             if (g.x == 0.0) continue;
             const int2 pq = round_robin_pair(n, r, k);
-            warp_rotate(colA(pq.x), colA(pq.y), m, V + (size_t)pq.x * n, V + (size_t)pq.y * n, n, lane, g.x, g.y);
+            warp_rotate<NJ, kApart>(colA(pq.x), colA(pq.y), m, V + (size_t)pq.x * n, V + (size_t)pq.y * n, n, lane, g.x,
+                                    g.y);
         }
         __syncthreads();
+    }
+}
+
+// What a kernel knows about its members' rows: nothing, at most kLanes, at
+// most kLanes / 2, or that they vary (the loops for every bound in one kernel,
+// which costs the longest of them their registers).
+enum BatchRows { kRowsAny, kRows256, kRows128, kRowsVary };
+
+__host__ __device__ constexpr BatchRows batch_rows(int m)
+{
+    return m <= kLanes / 2 ? kRows128 : (m <= kLanes ? kRows256 : kRowsAny);
+}
+
+// The same with the rows known as far as kRows says; true when some pair
+// rotated.  s_rot must be 0 on entry and is 0 again on return.
+template <BatchRows kRows, bool kApart, class ColA>
+__device__ __forceinline__ bool batch_sweep(ColA colA, double *V, int m, int n, double eps, double *st_pp,
+                                            double *st_qq, double *st_pq, double2 *st_cs, int &s_rot)
+{
+    constexpr bool kFew = kRows == kRows128 || kRows == kRowsVary;
+    constexpr bool kMany = kRows == kRowsVary;
+    if constexpr (kRows == kRowsAny) {
+        sweep_rounds<0, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+    } else if constexpr (!kFew) {
+        sweep_rounds<8, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+    } else {
+        if (m <= 32) sweep_rounds<1, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+        else if (m <= 64) sweep_rounds<2, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+        else if (!kMany || m <= 128) sweep_rounds<4, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+        else if (m <= 256) sweep_rounds<kMany ? 8 : 4, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+        else sweep_rounds<kMany ? 0 : 4, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
     }
     const bool any = s_rot != 0;
     __syncthreads();  // every thread has read the flag before it is reset
@@ -178,7 +288,7 @@ __device__ __forceinline__ bool batch_sweep(ColA colA, double *V, int m, int n, 
     return any;
 }
 
-template <bool kAShared, bool kVShared>
+template <bool kAShared, bool kVShared, BatchRows kRows>
 __global__ void __launch_bounds__(512) batch_kernel(const BatchDesc *__restrict__ descs, int count,
                                                     int *__restrict__ next, const void *__restrict__ a_all,
                                                     int a_is_f32, double eps, int max_sweeps,
@@ -234,45 +344,10 @@ __global__ void __launch_bounds__(512) batch_kernel(const BatchDesc *__restrict_
         for (size_t e = threadIdx.x; e < (size_t)n * n; e += blockDim.x) V[e] = (e / n == e % n) ? 1.0 : 0.0;
         if (threadIdx.x == 0) s_rot = 0;
         __syncthreads();
-        const int ne = n + (n & 1);
-        const int rounds = n >= 2 ? ne - 1 : 0;
-        const int npairs = n / 2;
         int sweeps = 1;
-        if (rounds > 0) {
+        if (n >= 2) {
             for (int sw = 0; sw < max_sweeps; ++sw) {
-                for (int r = 0; r < rounds; ++r) {
-                    // phase 1: dot products, one warp per pair
-                    for (int k = warp; k < npairs; k += nwarps) {
-                        const int2 pq = round_robin_pair(n, r, k);
-                        double pp, qq, pqv;
-                        warp_pair_stats(colA(pq.x), colA(pq.y), m, lane, pp, qq, pqv);
-                        if (lane == 0) {
-                            st_pp[k] = pp;
-                            st_qq[k] = qq;
-                            st_pq[k] = pqv;
-                        }
-                    }
-                    __syncthreads();
-                    // phase 2: angles, one thread per pair
-                    for (int k = threadIdx.x; k < npairs; k += blockDim.x) {
-                        double c, s;
-                        if (rotation_params(st_pp[k], st_qq[k], st_pq[k], eps, c, s)) s_rot = 1;
-                        st_cs[k] = make_double2(c, s);
-                    }
-                    __syncthreads();
-                    // phase 3: rotations, one warp per pair
-                    for (int k = warp; k < npairs; k += nwarps) {
-                        const double2 g = st_cs[k];
-                        if (g.x == 0.0) continue;
-                        const int2 pq = round_robin_pair(n, r, k);
-                        warp_rotate(colA(pq.x), colA(pq.y), m, V + (size_t)pq.x * n,
-                                    V + (size_t)pq.y * n, n, lane, g.x, g.y);
-                    }
-                    __syncthreads();
-                }
-                const bool any = s_rot != 0;
-                __syncthreads();  // every thread has read the flag before it is reset
-                if (threadIdx.x == 0) s_rot = 0;
+                const bool any = batch_sweep<kRows, kAShared && kVShared>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
                 sweeps = sw + 1;
                 if (!any) break;
             }
@@ -338,7 +413,7 @@ __global__ void __launch_bounds__(256, 2) batch_step_kernel(const StepDesc *__re
     if (threadIdx.x == 0) s_rot = 0;
     __syncthreads();
     bool any = false;
-    if (n >= 2) any = batch_sweep([&](int c) { return A + (size_t)c * m; }, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+    if (n >= 2) any = batch_sweep<kRowsVary, kVShared>([&](int c) { return A + (size_t)c * m; }, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
     for (size_t e = threadIdx.x; e < mn; e += blockDim.x) gA[e] = A[e];
     if (kVShared)
         for (size_t e = threadIdx.x; e < nn; e += blockDim.x) gV[e] = V[e];
@@ -391,15 +466,29 @@ __global__ void __launch_bounds__(256) batch_finish_kernel(const StepDesc *__res
 // (n), rotated together.  Pair arithmetic is batch_kernel's (warp-per-pair
 // dot products in the T = 256 order, Rutishauser angle, rot_p / rot_q), so
 // every member stays bit-identical to the plain path.
+//
+// What bounds it (B200, 228 x 189 members on 8 CTAs of 12 slots): one member
+// alone takes 2.9 us per round, a chain of dot products (0.5 us), angle (0.5),
+// rotation (0.8, at the shared-memory port's rate) and the cluster barrier; two
+// members on the same SMs take 3.0 us for both.  So a cluster is chosen such
+// that two of its CTAs share an SM where the member allows it.  Registers decide
+// the rest: at two CTAs per SM a thread has 80, and with the member's shape and
+// the ring indices of every buffer kept in them the loops' own values went to
+// local memory (5.2 us per round; in shared memory now, ClusterRound).  100
+// members: 21.5 ms, 31.3 on one CTA each; an SM per CTA with two slots in half
+// of its warps took 29.
 
-constexpr int kClusterThreads = 512;
-constexpr int kClusterSlotsPerWarp = 4;  // a CTA holds at most 4 * 16 pair slots
+// Threads of a cluster CTA with an SM to itself, and of one that shares it
+// with a CTA of another cluster.
+constexpr int kClusterThreads = 512, kClusterThreadsShared = 384;
+constexpr int kClusterMaxSlots = 64;  // pair slots per CTA
 
 __host__ __device__ constexpr int cluster_slots_max(int n, int C) { return ((n + (n & 1)) / 2 + C - 1) / C; }
 
-// Column buffer length: A's m rows, then V's n rows, padded to whole warps
-// (the padding rows are rotated and moved like the others and never read).
-__host__ __device__ constexpr int cluster_ld(int m, int n) { return (m + n + 31) & ~31; }
+// Column buffer length: A's m rows, then V's n rows, each padded to whole warps
+// (the padding rows are rotated and moved like the others; A's are zero).
+__host__ __device__ constexpr int cluster_rows(int m) { return (m + 31) & ~31; }
+__host__ __device__ constexpr int cluster_ld(int m, int n) { return cluster_rows(m) + cluster_rows(n); }
 
 // Shared memory of one CTA: column 0's fixed buffer and two rings.
 __host__ __device__ constexpr size_t cluster_smem_bytes(int m, int n, int C)
@@ -428,181 +517,320 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, double v)
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
 
-// Rotation of a column pair held in this CTA's buffers (x, y: ld rows, a
-// multiple of 32), written to (xo, yo): shared::cluster addresses of the same
-// buffers or of a neighbour's.  Every 256-row chunk is loaded before it is
-// stored, so in-place use is safe.  c = 0: the columns are only moved.
-__device__ __forceinline__ void warp_rotate_cl(const double *x, const double *y, uint32_t xo, uint32_t yo, int ld,
-                                               int lane, double c, double s, bool rotate)
-{
-    int r0 = 0;
-    for (; r0 + kLanes <= ld; r0 += kLanes) {
-        double xa[kW], ya[kW];
-#pragma unroll
-        for (int j = 0; j < kW; ++j) {
-            xa[j] = x[r0 + 32 * j + lane];
-            ya[j] = y[r0 + 32 * j + lane];
-        }
-#pragma unroll
-        for (int j = 0; j < kW; ++j) {
-            const uint32_t off = 8u * (uint32_t)(r0 + 32 * j + lane);
-            st_cluster(xo + off, rotate ? rot_p(c, s, xa[j], ya[j]) : xa[j]);
-            st_cluster(yo + off, rotate ? rot_q(c, s, xa[j], ya[j]) : ya[j]);
-        }
-    }
-    for (; r0 < ld; r0 += 32) {
-        const double xv = x[r0 + lane], yv = y[r0 + lane];
-        const uint32_t off = 8u * (uint32_t)(r0 + lane);
-        st_cluster(xo + off, rotate ? rot_p(c, s, xv, yv) : xv);
-        st_cluster(yo + off, rotate ? rot_q(c, s, xv, yv) : yv);
-    }
-}
-
 // Moves one column (ld rows) to a shared::cluster address.
 __device__ __forceinline__ void warp_move_cl(const double *x, uint32_t xo, int ld, int lane)
 {
     for (int r = lane; r < ld; r += 32) st_cluster(xo + 8u * (uint32_t)r, x[r]);
 }
 
-template <int C>
-__global__ void __launch_bounds__(kClusterThreads, 1)
+// Rotation of a column pair in this CTA's buffers (ld rows, a multiple of 32),
+// in place, four chunks loaded before any is stored.
+__device__ __forceinline__ void warp_rotate_local(double *x, double *y, int ld, int lane, double c, double s)
+{
+    x += lane;
+    y += lane;
+    int r = 0;
+    for (; r + 128 <= ld; r += 128) {
+        double xv[4], yv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            xv[j] = x[r + 32 * j];
+            yv[j] = y[r + 32 * j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            x[r + 32 * j] = rot_p(c, s, xv[j], yv[j]);
+            y[r + 32 * j] = rot_q(c, s, xv[j], yv[j]);
+        }
+    }
+    double xv[3], yv[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        if (r + 32 * j < ld) {
+            xv[j] = x[r + 32 * j];
+            yv[j] = y[r + 32 * j];
+        }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        if (r + 32 * j < ld) {
+            x[r + 32 * j] = rot_p(c, s, xv[j], yv[j]);
+            y[r + 32 * j] = rot_q(c, s, xv[j], yv[j]);
+        }
+}
+
+// The same to the shared::cluster addresses xo and yo of the columns' next
+// buffers.
+__device__ __forceinline__ void warp_rotate_away(const double *x, const double *y, uint32_t xo, uint32_t yo, int ld,
+                                                 int lane, double c, double s)
+{
+    x += lane;
+    y += lane;
+    xo += 8u * (uint32_t)lane;
+    yo += 8u * (uint32_t)lane;
+    int r = 0;
+    for (; r + 128 <= ld; r += 128) {
+        double xv[4], yv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            xv[j] = x[r + 32 * j];
+            yv[j] = y[r + 32 * j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            st_cluster(xo + 8u * (uint32_t)(r + 32 * j), rot_p(c, s, xv[j], yv[j]));
+            st_cluster(yo + 8u * (uint32_t)(r + 32 * j), rot_q(c, s, xv[j], yv[j]));
+        }
+    }
+    for (; r < ld; r += 32) {
+        const double xv = x[r], yv = y[r];
+        st_cluster(xo + 8u * (uint32_t)r, rot_p(c, s, xv, yv));
+        st_cluster(yo + 8u * (uint32_t)r, rot_q(c, s, xv, yv));
+    }
+}
+
+// Angle of a slot's pair of columns (mp rows of A in whole chunks, padded with
+// zeros; m real ones); false when it does not rotate.  kTall: more than kLanes
+// rows.
+template <bool kTall>
+__device__ __forceinline__ bool warp_angle_cl(const double *x, const double *y, int m, int mp, int lane, double eps,
+                                              double &c, double &s)
+{
+    double total;
+    if constexpr (kTall) {
+        total = warp_pair_stats<0>(x, y, m, lane);
+    } else {
+        double xr[kW], yr[kW];
+#pragma unroll
+        for (int j = 0; j < kW; ++j) {
+            const bool in = 32 * j < mp;
+            xr[j] = in ? x[32 * j + lane] : 0.0;
+            yr[j] = in ? y[32 * j + lane] : 0.0;
+        }
+        // the register levels of the tree, s[j] += s[j + 4], + 2, + 1, one sum
+        // after the other
+        auto sum = [](const double(&a)[kW], const double(&b)[kW]) {
+            return ((a[0] * b[0] + a[4] * b[4]) + (a[2] * b[2] + a[6] * b[6])) +
+                   ((a[1] * b[1] + a[5] * b[5]) + (a[3] * b[3] + a[7] * b[7]));
+        };
+        total = warp_tree3(sum(xr, xr), sum(yr, yr), sum(xr, yr), lane);
+    }
+    const double pp = __shfl_sync(0xffffffffu, total, 0);
+    const double pq = __shfl_sync(0xffffffffu, total, 8);
+    const double qq = __shfl_sync(0xffffffffu, total, 16);
+    // Far below the threshold (by a factor of two, well above the rounding of
+    // either side) nothing rotates: most pairs of the last sweeps stop here.
+    if (pq * pq < (0.25 * eps * eps) * (fmax(pp, 0.0) * fmax(qq, 0.0))) return false;
+    return rotation_params(pp, qq, pq, eps, c, s);
+}
+
+// A CTA's share of a member: its slots [k0, k0 + S) of the circle's half, and
+// its buffers (offsets in doubles): column 0's fixed one (CTA 0 only, where slot
+// 0's top never moves: jt0 = 1), the top ring of rt buffers and the bottom ring
+// of rb.  Top slot j is in top buffer (j - jt0 - g) mod rt at round g, bottom
+// slot j in bottom buffer (j + g) mod rb.
+struct ClusterShare {
+    int m, n, ne, half, L, ld, mp, k0, S, jt0, rt, rb, top_off, bot_off;
+    __device__ ClusterShare(int m_, int n_, int rank, int C) : m(m_), n(n_)
+    {
+        ne = n + (n & 1);
+        half = ne / 2;
+        L = ne - 1;
+        ld = cluster_ld(m, n);
+        mp = cluster_rows(m);
+        k0 = rank * half / C;
+        S = (rank + 1) * half / C - k0;  // >= 2 (host: half >= 2C)
+        jt0 = rank == 0 ? 1 : 0;
+        rt = S - jt0 + 1;
+        rb = S + 1;
+        top_off = ld;
+        bot_off = (cluster_slots_max(n, C) + 2) * ld;
+    }
+    __device__ int top_at(int j, int g) const { return jt0 && j == 0 ? 0 : top_off + pmod(j - jt0 - g, rt) * ld; }
+    __device__ int bot_at(int j, int g) const { return bot_off + pmod(j + g, rb) * ld; }
+};
+
+// What a round needs besides: g modulo the rings' lengths, the slot of this CTA
+// that holds the dummy column of an odd n (or -1) and in which position, and
+// the shared::cluster addresses that the last slot's top column and the first
+// slot's bottom column move to.  One thread works it out a round ahead, in
+// shared memory: kept in every thread's registers, this and the member's shape
+// pushed the loops' own values into local memory.
+struct ClusterRound {
+    int gt, gb, dummy, dummy_top;
+    uint32_t top_to, bot_to;
+};
+struct ClusterKeep {
+    int idx, m, n;     // the member
+    int dpos;          // circle position of the dummy column
+    int o_top, o_bot;  // ring buffers that receive this CTA's outgoing columns
+    int s_right, s_left;
+};
+
+__device__ __forceinline__ void cluster_round(const ClusterShare &sh, int rank, int C, const ClusterKeep &kp,
+                                              uint32_t self, uint32_t right, uint32_t left, int gt, int gb,
+                                              ClusterRound &out)
+{
+    out.gt = gt;
+    out.gb = gb;
+    out.dummy_top = kp.dpos < sh.half;
+    const int d = (out.dummy_top ? kp.dpos : sh.L - kp.dpos) - sh.k0;
+    out.dummy = (sh.n & 1) && d >= 0 && d < sh.S ? d : -1;
+    out.top_to = rank < C - 1 ? right + 8u * (uint32_t)(sh.top_off + kp.o_top * sh.ld)
+                              : self + 8u * (uint32_t)(sh.bot_off + kp.o_top * sh.ld);
+    out.bot_to = rank > 0 ? left + 8u * (uint32_t)(sh.bot_off + kp.o_bot * sh.ld)
+                          : self + 8u * (uint32_t)(sh.top_off + kp.o_bot * sh.ld);
+}
+
+// A member's descriptor, read anew each time (not kept in registers).
+__device__ __forceinline__ BatchDesc read_desc(const BatchDesc *descs, int idx)
+{
+    const volatile BatchDesc *p = descs + idx;
+    BatchDesc d;
+    d.m = p->m;
+    d.n = p->n;
+    d.a_off = p->a_off;
+    d.s_off = p->s_off;
+    d.v_off = p->v_off;
+    d.u_off = p->u_off;
+    return d;
+}
+
+template <int C, bool kTall, bool kShare>
+__global__ void __launch_bounds__(kShare ? kClusterThreadsShared : kClusterThreads, kShare ? 2 : 1)
     batch_cluster_kernel(const BatchDesc *__restrict__ descs, int count, int *__restrict__ next,
                          const void *__restrict__ a_all, int a_is_f32, double eps, int max_sweeps,
                          double *__restrict__ sigma_all, double *__restrict__ v_all, double *__restrict__ u_all,
                          int *__restrict__ sweeps_all)
 {
     namespace cg = cooperative_groups;
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     __shared__ int s_idx;
     __shared__ int s_rot;
     __shared__ unsigned long long s_stamp;  // rank 0's copy: last (member, sweep) stamp that rotated
+    __shared__ ClusterKeep s_keep;
+    __shared__ __align__(16) ClusterRound s_round[2];  // by round parity
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int *idx0 = cluster.map_shared_rank(&s_idx, 0);
-    unsigned long long *stamp0 = cluster.map_shared_rank(&s_stamp, 0);
-    // shared::cluster addresses of the start of the dynamic shared memory:
-    // this CTA's own and its neighbours' (same layout in every CTA)
-    const uint32_t sm_self = cluster_addr(smem, rank);
-    const uint32_t sm_right = cluster_addr(smem, rank < C - 1 ? rank + 1 : rank);
-    const uint32_t sm_left = cluster_addr(smem, rank > 0 ? rank - 1 : rank);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int nwarps = (kShare ? kClusterThreadsShared : kClusterThreads) / 32;
+    constexpr int kKeeper = 64;  // the thread that looks a round ahead
     if (threadIdx.x == 0) {
         s_rot = 0;
         s_stamp = 0;
     }
     for (;;) {
-        if (rank == 0 && threadIdx.x == 0) s_idx = atomicAdd(next, 1);
-        cluster.sync();  // (the first one also orders the initialisation above)
-        const int idx = *(volatile const int *)idx0;
-        // every CTA has read the index and finished the previous member's
-        // outputs before any CTA writes into another's buffers or exits
-        cluster.sync();
-        if (idx >= count) return;
-        const BatchDesc d = descs[idx];
-        const int m = d.m, n = d.n;
-        const int ne = n + (n & 1), half = ne / 2, L = ne - 1;
-        const int rounds = n >= 2 ? L : 0;
-        const int ld = cluster_ld(m, n);
-        const int smax = cluster_slots_max(n, C);
-        const int k0 = rank * half / C, k1 = (rank + 1) * half / C, S = k1 - k0;  // S >= 2 (host: half >= 2C)
-        // buffers (offsets in doubles): column 0's fixed one (CTA 0 only), the
-        // top ring, the bottom ring
-        const int top_off = ld, bot_off = (smax + 2) * ld;
-        const int jt0 = rank == 0 ? 1 : 0;  // first top slot that moves
-        const int rt = S - jt0 + 1, rb = S + 1;
-        const int s_right = rank < C - 1 ? (rank + 2) * half / C - k1 : 0;
-        const int s_left = rank > 0 ? k0 - (rank - 1) * half / C : 0;
-        // top slot j is in top buffer (j - jt0 - g) mod rt at round g, bottom
-        // slot j in bottom buffer (j + g) mod rb
-        auto top_at = [&](int j, int g) { return (rank == 0 && j == 0) ? 0 : top_off + pmod(j - jt0 - g, rt) * ld; };
-        auto bot_at = [&](int j, int g) { return bot_off + pmod(j + g, rb) * ld; };
-        // round 0: position p holds column p; V = I
-        const int ncl = 2 * S;
-        for (int e = threadIdx.x; e < m * ncl; e += blockDim.x) {
-            const int row = e / ncl, cc = e - row * ncl;
-            const int j = cc < S ? cc : cc - S;
-            const int col = cc < S ? k0 + j : ne - 1 - (k0 + j);
-            if (col >= n) continue;  // the dummy column of an odd n
-            const size_t src = (size_t)d.a_off + (size_t)row * n + col;
-            smem[(cc < S ? top_at(j, 0) : bot_at(j, 0)) + row] =
-                a_is_f32 ? (double)reinterpret_cast<const float *>(a_all)[src]
-                         : reinterpret_cast<const double *>(a_all)[src];
-        }
-        for (int e = threadIdx.x; e < n * ncl; e += blockDim.x) {
-            const int row = e / ncl, cc = e - row * ncl;
-            const int j = cc < S ? cc : cc - S;
-            const int col = cc < S ? k0 + j : ne - 1 - (k0 + j);
-            if (col >= n) continue;
-            smem[(cc < S ? top_at(j, 0) : bot_at(j, 0)) + m + row] = row == col ? 1.0 : 0.0;
+        int ld, mp, m, rounds, S, jt0, bot_base;
+        {
+            const int rank = (int)cluster.block_rank();
+            if (rank == 0 && threadIdx.x == 0) s_idx = atomicAdd(next, 1);
+            cluster.sync();  // (the first one also orders the initialisation above)
+            const int idx = *(volatile const int *)cluster.map_shared_rank(&s_idx, 0);
+            // every CTA has read the index and finished the previous member's
+            // outputs before any CTA writes into another's buffers or exits
+            cluster.sync();
+            if (idx >= count) return;
+            const BatchDesc d = read_desc(descs, idx);
+            const ClusterShare sh(d.m, d.n, rank, C);
+            // round 0: position p holds column p; V = I
+            const int ncl = 2 * sh.S;
+            for (int e = threadIdx.x; e < sh.mp * ncl; e += blockDim.x) {
+                const int row = e / ncl, cc = e - row * ncl;
+                const int j = cc < sh.S ? cc : cc - sh.S;
+                const int col = cc < sh.S ? sh.k0 + j : sh.ne - 1 - (sh.k0 + j);
+                if (col >= sh.n) continue;  // the dummy column of an odd n
+                const size_t src = (size_t)d.a_off + (size_t)row * sh.n + col;
+                smem[(cc < sh.S ? sh.top_at(j, 0) : sh.bot_at(j, 0)) + row] =
+                    row >= sh.m ? 0.0
+                                : (a_is_f32 ? (double)reinterpret_cast<const float *>(a_all)[src]
+                                            : reinterpret_cast<const double *>(a_all)[src]);
+            }
+            for (int e = threadIdx.x; e < (sh.ld - sh.mp) * ncl; e += blockDim.x) {
+                const int row = e / ncl, cc = e - row * ncl;
+                const int j = cc < sh.S ? cc : cc - sh.S;
+                const int col = cc < sh.S ? sh.k0 + j : sh.ne - 1 - (sh.k0 + j);
+                if (col >= sh.n) continue;
+                smem[(cc < sh.S ? sh.top_at(j, 0) : sh.bot_at(j, 0)) + sh.mp + row] = row == col ? 1.0 : 0.0;
+            }
+            if (threadIdx.x == kKeeper) {
+                // the right neighbour's spare top buffer (the last CTA: its own
+                // spare bottom one) and the left neighbour's spare bottom buffer
+                // (CTA 0: its own spare top one)
+                s_keep.idx = idx;
+                s_keep.m = d.m;
+                s_keep.n = d.n;
+                s_keep.dpos = sh.L;
+                s_keep.s_right = rank < C - 1 ? (rank + 2) * sh.half / C - (rank + 1) * sh.half / C : 0;
+                s_keep.s_left = rank > 0 ? sh.k0 - (rank - 1) * sh.half / C : 0;
+                s_keep.o_top = rank < C - 1 ? s_keep.s_right : sh.S;
+                s_keep.o_bot = rank > 0 ? s_keep.s_left : sh.rt - 1;
+                cluster_round(sh, rank, C, s_keep, cluster_addr(smem, rank),
+                              cluster_addr(smem, rank < C - 1 ? rank + 1 : rank),
+                              cluster_addr(smem, rank > 0 ? rank - 1 : rank), 0, 0, s_round[0]);
+            }
+            ld = sh.ld;
+            mp = sh.mp;
+            m = sh.m;
+            S = sh.S;
+            jt0 = sh.jt0;
+            bot_base = sh.bot_off;
+            rounds = sh.n >= 2 ? sh.L : 0;
         }
         __syncthreads();
-        // This warp's slots j = warp + t * nwarps, tracked from round to round:
-        // the circle values at their two positions (n = the dummy) and their
-        // ring buffers.  Position values fall by one per round (1 -> L).
-        int pv[kClusterSlotsPerWarp], qv[kClusterSlotsPerWarp], tb[kClusterSlotsPerWarp], bb[kClusterSlotsPerWarp];
-#pragma unroll
-        for (int t = 0; t < kClusterSlotsPerWarp; ++t) {
-            const int j = warp + t * nwarps, k = k0 + j;
-            pv[t] = k;
-            qv[t] = ne - 1 - k;
-            tb[t] = (rank == 0 && j == 0) ? -1 : j - jt0;
-            bb[t] = j;
-        }
-        // ring buffers that receive this CTA's outgoing columns in round g:
-        // the right neighbour's spare top buffer (the last CTA: its own spare
-        // bottom one) and the left neighbour's spare bottom buffer (CTA 0: its
-        // own spare top one)
-        int o_top = rank < C - 1 ? s_right : S;
-        int o_bot = rank > 0 ? s_left : rt - 1;
         int g = 0, sweeps = 1;
         if (rounds > 0) {
             for (int sw = 0; sw < max_sweeps; ++sw) {
                 for (int r = 0; r < rounds; ++r, ++g) {
-#pragma unroll
-                    for (int t = 0; t < kClusterSlotsPerWarp; ++t) {
-                        const int j = warp + t * nwarps;
-                        if (j < S) {
-                            const int xo = tb[t] < 0 ? 0 : top_off + tb[t] * ld;
-                            const int yo = bot_off + bb[t] * ld;
-                            const double *xt = smem + xo;
-                            const double *xb = smem + yo;
-                            const uint32_t dt = j == S - 1
-                                                    ? (rank < C - 1 ? sm_right + 8u * (uint32_t)(top_off + o_top * ld)
-                                                                    : sm_self + 8u * (uint32_t)(bot_off + o_top * ld))
-                                                    : sm_self + 8u * (uint32_t)xo;
-                            const uint32_t db = j == 0
-                                                    ? (rank > 0 ? sm_left + 8u * (uint32_t)(bot_off + o_bot * ld)
-                                                                : sm_self + 8u * (uint32_t)(top_off + o_bot * ld))
-                                                    : sm_self + 8u * (uint32_t)yo;
-                            const bool real = pv[t] != n && qv[t] != n;
-                            double c = 0.0, s = 0.0;
-                            if (real) {
-                                double pp, qq, pqv;
-                                warp_pair_stats(xt, xb, m, lane, pp, qq, pqv);
-                                if (lane == 0 && rotation_params(pp, qq, pqv, eps, c, s)) s_rot = 1;
-                                c = __shfl_sync(0xffffffffu, c, 0);
-                                s = __shfl_sync(0xffffffffu, s, 0);
-                            }
-                            if (c != 0.0) {
-                                warp_rotate_cl(xt, xb, dt, db, ld, lane, c, s, true);
-                            } else {  // no rotation (or the dummy's slot): the columns only move
-                                if (j == S - 1 && pv[t] != n) warp_move_cl(xt, dt, ld, lane);
-                                if (j == 0 && qv[t] != n) warp_move_cl(xb, db, ld, lane);
-                            }
-                            if (pv[t] != 0) pv[t] = pv[t] == 1 ? L : pv[t] - 1;
-                            qv[t] = qv[t] == 1 ? L : qv[t] - 1;
-                            if (tb[t] >= 0) tb[t] = tb[t] == 0 ? rt - 1 : tb[t] - 1;
-                            bb[t] = bb[t] == rb - 1 ? 0 : bb[t] + 1;
+                    const volatile ClusterRound &rd = s_round[g & 1];
+#pragma unroll 1
+                    for (int j = warp; j < S; j += nwarps) {
+                        int tb = j - jt0 - rd.gt, bb = j + rd.gb;
+                        if (tb < 0) tb += S - jt0 + 1;
+                        if (bb > S) bb -= S + 1;
+                        double *xt = smem + (jt0 && j == 0 ? 0 : (1 + tb) * ld);
+                        double *xb = smem + bot_base + bb * ld;
+                        const bool dummy = j == rd.dummy;
+                        double c, s;
+                        const bool rotates = !dummy && warp_angle_cl<kTall>(xt, xb, m, mp, lane, eps, c, s);
+                        if (rotates && lane == 0) s_rot = 1;
+                        if (j != 0 && j != S - 1) {
+                            if (rotates) warp_rotate_local(xt, xb, ld, lane, c, s);
+                            continue;
+                        }
+                        // a slot at the end of the CTA's row: its outer column
+                        // leaves (at either end of the circle into the other
+                        // ring), rotated or (the dummy's slot too) as it is
+                        const uint32_t sm_self = cluster_addr(smem, (int)cluster.block_rank());
+                        const uint32_t dt =
+                            j == S - 1 ? rd.top_to : sm_self + (uint32_t)((const char *)xt - (const char *)smem);
+                        const uint32_t db = j == 0 ? rd.bot_to : sm_self + (uint32_t)((const char *)xb - (const char *)smem);
+                        if (rotates) {
+                            warp_rotate_away(xt, xb, dt, db, ld, lane, c, s);
+                        } else {
+                            if (j == S - 1 && !(dummy && rd.dummy_top)) warp_move_cl(xt, dt, ld, lane);
+                            if (j == 0 && !(dummy && !rd.dummy_top)) warp_move_cl(xb, db, ld, lane);
                         }
                     }
-                    if (rank < C - 1) o_top = o_top == 0 ? s_right : o_top - 1;
-                    else o_top = o_top == rb - 1 ? 0 : o_top + 1;
-                    if (rank > 0) o_bot = o_bot == s_left ? 0 : o_bot + 1;
-                    else o_bot = o_bot == 0 ? rt - 1 : o_bot - 1;
+                    if (threadIdx.x == kKeeper) {
+                        const int rank = (int)cluster.block_rank();
+                        ClusterKeep kp = s_keep;
+                        const ClusterShare sh(kp.m, kp.n, rank, C);
+                        kp.dpos = kp.dpos == sh.L ? 1 : kp.dpos + 1;
+                        if (rank < C - 1) kp.o_top = kp.o_top == 0 ? kp.s_right : kp.o_top - 1;
+                        else kp.o_top = kp.o_top == sh.rb - 1 ? 0 : kp.o_top + 1;
+                        if (rank > 0) kp.o_bot = kp.o_bot == kp.s_left ? 0 : kp.o_bot + 1;
+                        else kp.o_bot = kp.o_bot == 0 ? sh.rt - 1 : kp.o_bot - 1;
+                        s_keep = kp;
+                        cluster_round(sh, rank, C, kp, cluster_addr(smem, rank),
+                                      cluster_addr(smem, rank < C - 1 ? rank + 1 : rank),
+                                      cluster_addr(smem, rank > 0 ? rank - 1 : rank),
+                                      rd.gt == sh.rt - 1 ? 0 : rd.gt + 1, rd.gb == sh.rb - 1 ? 0 : rd.gb + 1,
+                                      s_round[(g + 1) & 1]);
+                    }
                     cluster.sync();
                 }
                 // sweep test over the cluster: a CTA that rotated raises rank 0's stamp
-                const unsigned long long stamp = (unsigned long long)idx * (unsigned)(max_sweeps + 1) + sw + 1;
+                unsigned long long *stamp0 = cluster.map_shared_rank(&s_stamp, 0);
+                const unsigned long long stamp =
+                    (unsigned long long)*(volatile int *)&s_keep.idx * (unsigned)(max_sweeps + 1) + sw + 1;
                 if (threadIdx.x == 0) {
                     if (s_rot) atomicMax(stamp0, stamp);
                     s_rot = 0;
@@ -614,21 +842,25 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
             }
         }
         // every sweep is a whole turn of the circle: position p holds column p again
+        const int rank = (int)cluster.block_rank();
+        const int idx = *(volatile int *)&s_keep.idx;
+        const BatchDesc d = read_desc(descs, idx);
+        const ClusterShare sh(d.m, d.n, rank, C);
         double *sg = sigma_all + d.s_off;
-        for (int cc = warp; cc < ncl; cc += nwarps) {
-            const int j = cc < S ? cc : cc - S;
-            const int col = cc < S ? k0 + j : ne - 1 - (k0 + j);
-            if (col >= n) continue;
-            const double *x = smem + (cc < S ? top_at(j, g) : bot_at(j, g));
-            const double sc = sqrt(fmax(warp_norm2(x, m, lane), 0.0));
+        for (int cc = warp; cc < 2 * sh.S; cc += nwarps) {
+            const int j = cc < sh.S ? cc : cc - sh.S;
+            const int col = cc < sh.S ? sh.k0 + j : sh.ne - 1 - (sh.k0 + j);
+            if (col >= sh.n) continue;
+            const double *x = smem + (cc < sh.S ? sh.top_at(j, g) : sh.bot_at(j, g));
+            const double sc = sqrt(fmax(warp_norm2(x, sh.m, lane), 0.0));
             if (lane == 0) sg[col] = sc;
             if (u_all != nullptr) {
                 double *u = u_all + d.u_off;
-                for (int i = lane; i < m; i += 32) u[(size_t)i * n + col] = (sc > eps) ? (x[i] / sc) : 0.0;
+                for (int i = lane; i < sh.m; i += 32) u[(size_t)i * sh.n + col] = (sc > eps) ? (x[i] / sc) : 0.0;
             }
             if (v_all != nullptr) {
                 double *vo = v_all + d.v_off;
-                for (int i = lane; i < n; i += 32) vo[(size_t)i * n + col] = x[m + i];
+                for (int i = lane; i < sh.n; i += 32) vo[(size_t)i * sh.n + col] = x[sh.mp + i];
             }
         }
         if (rank == 0 && threadIdx.x == 0 && sweeps_all != nullptr) sweeps_all[idx] = sweeps;
@@ -638,34 +870,62 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
 using ClusterFn = void (*)(const BatchDesc *, int, int *, const void *, int, double, int, double *, double *, double *,
                            int *);
 
-ClusterFn cluster_fn(int C)
+template <bool kTall, bool kShare>
+ClusterFn cluster_fn_c(int C)
 {
-    return C == 2 ? batch_cluster_kernel<2> : (C == 4 ? batch_cluster_kernel<4> : batch_cluster_kernel<8>);
+    return C == 2 ? batch_cluster_kernel<2, kTall, kShare>
+                  : (C == 4 ? batch_cluster_kernel<4, kTall, kShare> : batch_cluster_kernel<8, kTall, kShare>);
+}
+
+// `tall`: members of more than kLanes rows; `share`: two CTAs per SM.
+ClusterFn cluster_fn(int C, bool tall, bool share)
+{
+    if (tall) return share ? cluster_fn_c<true, true>(C) : cluster_fn_c<true, false>(C);
+    return share ? cluster_fn_c<false, true>(C) : cluster_fn_c<false, false>(C);
 }
 
 // Size classes whose members go to clusters where one fits (bit c = class c;
 // classes 2-4 only), initially the compiled-in tuning table's choice.
 // Process-wide.
 #ifndef JSVD_BATCH_CLUSTER_CLASSES
-#define JSVD_BATCH_CLUSTER_CLASSES ((1 << 3) | (1 << 4))
+#define JSVD_BATCH_CLUSTER_CLASSES (1 << 4)
 #endif
 std::atomic<int> g_cluster_mask{JSVD_BATCH_CLUSTER_CLASSES};  // the tuning table's choice
 int batch_cluster_mask() { return g_cluster_mask.load(std::memory_order_relaxed); }
 
-// Smallest cluster (2, 4, 8 CTAs) whose shared memory holds an m x n member
-// with at least two and at most 64 pair slots per CTA; 0 when none does.
-int cluster_size_for(int m, int n, size_t smem_cap)
+// Cluster of an m x n member: the smallest (2, 4, 8 CTAs) in which two CTAs
+// share an SM's memory with at most one pair slot per warp (share), so that
+// one member's loads and stores run beside the other's arithmetic; else the
+// smallest that holds the member with an SM per CTA; 0 when none does.  At
+// least two slots per CTA.
+int cluster_size_for(int m, int n, size_t smem_cap, bool &share)
 {
     const int half = (n + (n & 1)) / 2;
+    share = true;
     for (int C : {2, 4, 8})
-        if (half >= 2 * C && cluster_slots_max(n, C) <= kClusterSlotsPerWarp * (kClusterThreads / 32) &&
-            cluster_smem_bytes(m, n, C) <= smem_cap)
+        if (half >= 2 * C && cluster_slots_max(n, C) <= kClusterThreadsShared / 32 &&
+            cluster_smem_bytes(m, n, C) <= smem_cap / 2 - 1024)
+            return C;
+    share = false;
+    for (int C : {2, 4, 8})
+        if (half >= 2 * C && cluster_slots_max(n, C) <= kClusterMaxSlots && cluster_smem_bytes(m, n, C) <= smem_cap)
             return C;
     return 0;
 }
 
 using BatchFn = void (*)(const BatchDesc *, int, int *, const void *, int, double, int, double *, double *,
                          double *, int *, double *, size_t, int);
+
+// The one-CTA kernel of a class and of members whose rows are known as far as
+// `rows` says.
+BatchFn batch_fn(int cls, BatchRows rows)
+{
+    if (cls <= 2)
+        return rows == kRows128 ? batch_kernel<true, true, kRows128>
+                                : (rows == kRows256 ? batch_kernel<true, true, kRows256> : batch_kernel<true, true, kRowsAny>);
+    if (cls == 3) return rows == kRowsAny ? batch_kernel<true, false, kRowsAny> : batch_kernel<true, false, kRows256>;
+    return rows == kRowsAny ? batch_kernel<false, false, kRowsAny> : batch_kernel<false, false, kRows256>;
+}
 
 // Per-thread timing events: whole call and one pair per size class.
 struct ThreadEvents {
@@ -776,7 +1036,6 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
         int threads;
         int ctas_per_sm;
         bool a_shared, v_shared;
-        BatchFn fn;
     };
     Class classes[kClasses];
     int max_ctas[kClasses] = {};
@@ -785,8 +1044,6 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
         classes[c].ctas_per_sm = kBuiltinTuning[c].ctas_per_sm;
         classes[c].a_shared = class_a_shared(c);
         classes[c].v_shared = class_v_shared(c);
-        classes[c].fn = c <= 2 ? batch_kernel<true, true>
-                               : (c == 3 ? batch_kernel<true, false> : batch_kernel<false, false>);
         max_ctas[c] = kBuiltinTuning[c].max_ctas;
     }
     if (req.tuning != nullptr) {
@@ -828,9 +1085,12 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
     // cluster mask), then the rest by the class's own kernel.  Largest work
     // first inside each group (tail balance of the work queue).
     struct Group {
-        int cls, csize, first, count;
+        int cls, csize;
+        bool tall, share;
+        BatchRows rows;
+        int first, count;
         size_t smem, gws;
-        int grid;
+        int grid, threads;
     };
     auto work = [&](int i) { return member_work(all[i].m, all[i].n); };
     const int mask = batch_cluster_mask();
@@ -841,14 +1101,21 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
     order_index.reserve(count);
     for (int c = kClasses - 1; c >= 0; --c) {
         std::sort(members[c].begin(), members[c].end(), [&](int x, int y) { return work(x) > work(y); });
-        std::vector<int> sub[4];  // own kernel, clusters of 2, 4, 8
+        // by kernel: own (0-2, by rows), clusters of 2, 4, 8 (3-5), + 3 sharing an
+        // SM, + 6 tall
+        std::vector<int> sub[15];
         for (int i : members[c]) {
-            const int C = ((mask >> c) & 1) ? cluster_size_for(all[i].m, all[i].n, smem_cap) : 0;
-            sub[C == 0 ? 0 : (C == 2 ? 1 : (C == 4 ? 2 : 3))].push_back(i);
+            bool share = false;
+            const int C = ((mask >> c) & 1) ? cluster_size_for(all[i].m, all[i].n, smem_cap, share) : 0;
+            const BatchRows rows = c <= 2 ? batch_rows(all[i].m) : std::min(batch_rows(all[i].m), kRows256);
+            sub[C == 0 ? (int)rows : (C == 2 ? 3 : (C == 4 ? 4 : 5)) + (share ? 3 : 0) + (all[i].m > kLanes ? 6 : 0)]
+                .push_back(i);
         }
-        for (int s : {3, 2, 1, 0}) {
+        for (int s : {14, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 0, 1, 2}) {
             if (sub[s].empty()) continue;
-            Group g{c, s == 0 ? 0 : (1 << s), (int)ordered.size(), (int)sub[s].size(), 0, 0, 0};
+            const int k = s < 3 ? 0 : s - 3;
+            Group g{c, s < 3 ? 0 : (1 << (k % 3 + 1)), s >= 3 && k >= 6, s >= 3 && k / 3 % 2 == 1, (BatchRows)std::min(s, 2),
+                    (int)ordered.size(), (int)sub[s].size(), 0, 0, 0, 0};
             for (int i : sub[s]) {
                 ordered.push_back(all[i]);
                 order_index.push_back(i);
@@ -870,7 +1137,7 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
     for (size_t k = 0; k < groups.size(); ++k) {
         Group &g = groups[k];
         if (g.csize > 0) {
-            JSVD_CUDA_TRY(cudaFuncSetAttribute(cluster_fn(g.csize), cudaFuncAttributeMaxDynamicSharedMemorySize,
+            JSVD_CUDA_TRY(cudaFuncSetAttribute(cluster_fn(g.csize, g.tall, g.share), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)smem_cap));
             cudaLaunchConfig_t lc = {};
             cudaLaunchAttribute at[1];
@@ -879,12 +1146,12 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
             at[0].val.clusterDim.y = 1;
             at[0].val.clusterDim.z = 1;
             lc.gridDim = dim3((unsigned)g.csize);
-            lc.blockDim = dim3(kClusterThreads);
+            lc.blockDim = dim3(g.share ? kClusterThreadsShared : kClusterThreads);
             lc.dynamicSmemBytes = g.smem;
             lc.attrs = at;
             lc.numAttrs = 1;
             int clusters = 0;
-            JSVD_CUDA_TRY(cudaOccupancyMaxActiveClusters(&clusters, cluster_fn(g.csize), &lc));
+            JSVD_CUDA_TRY(cudaOccupancyMaxActiveClusters(&clusters, cluster_fn(g.csize, g.tall, g.share), &lc));
             if (clusters <= 0) {
                 set_last_error(JSVD_ERR_RUNTIME, "No cluster of the batched solver fits the device.");
                 return JSVD_ERR_RUNTIME;
@@ -892,7 +1159,20 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
             g.grid = std::min(g.count, clusters) * g.csize;
         } else {
             const Class &cl = classes[g.cls];
-            g.grid = std::min(g.count, sms * cl.ctas_per_sm);
+            g.threads = cl.threads;
+            int ctas_per_sm = cl.ctas_per_sm;
+            // The table's shapes suit many members per resident CTA.  Up to one
+            // and a half, the last ones decide: half as many CTAs of twice the
+            // warps (740 members of class 0: 4.5 -> 3.1 ms, 365 of class 1: 8.4
+            // -> 6.2; at five per CTA and more the table's are the faster, 4.1
+            // -> 3.3 ms for 2921 members), and a CTA to itself for every member
+            // when the SMs suffice (79 of class 1: 2.2 -> 1.8 ms).
+            if (req.tuning == nullptr && 2 * g.count <= 3 * sms * ctas_per_sm && ctas_per_sm > 1) {
+                const int share = g.count <= sms ? ctas_per_sm : 2;
+                g.threads = std::min(512, g.threads * share);
+                ctas_per_sm = std::max(1, ctas_per_sm / share);
+            }
+            g.grid = std::min(g.count, sms * ctas_per_sm);
             if (max_ctas[g.cls] > 0) g.grid = std::min(g.grid, max_ctas[g.cls]);
             gws_base[k] = gws_total;
             gws_total += g.gws * (size_t)g.grid;
@@ -916,9 +1196,10 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
     JSVD_CUDA_TRY(cudaMemcpyAsync(d_desc, ordered.data(), sizeof(BatchDesc) * ordered.size(), cudaMemcpyHostToDevice,
                                   stream));
     JSVD_CUDA_TRY(cudaMemsetAsync(d_next, 0, sizeof(int) * ngroups, stream));
-    for (BatchFn fn : {(BatchFn)batch_kernel<true, true>, (BatchFn)batch_kernel<true, false>,
-                       (BatchFn)batch_kernel<false, false>})
-        JSVD_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
+    for (int c : {2, 3, 4})
+        for (BatchRows rows : {kRowsAny, kRows256, kRows128})
+            JSVD_CUDA_TRY(cudaFuncSetAttribute(batch_fn(c, rows), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem_cap));
     JSVD_CUDA_TRY(cudaEventRecord(ts->t0, stream));
     int launches = 0;
     std::vector<int> class_count(kClasses, 0);
@@ -939,19 +1220,19 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
             at[0].val.clusterDim.y = 1;
             at[0].val.clusterDim.z = 1;
             lc.gridDim = dim3((unsigned)g.grid);
-            lc.blockDim = dim3(kClusterThreads);
+            lc.blockDim = dim3(g.share ? kClusterThreadsShared : kClusterThreads);
             lc.dynamicSmemBytes = g.smem;
             lc.stream = stream;
             lc.attrs = at;
             lc.numAttrs = 1;
-            JSVD_CUDA_TRY(cudaLaunchKernelEx(&lc, cluster_fn(g.csize), (const BatchDesc *)(d_desc + g.first), g.count,
+            JSVD_CUDA_TRY(cudaLaunchKernelEx(&lc, cluster_fn(g.csize, g.tall, g.share), (const BatchDesc *)(d_desc + g.first), g.count,
                                              d_next + k, req.a, req.a_is_f32, req.eps, req.max_sweeps, req.sigma,
                                              req.v, req.u, d_sweeps + g.first));
         } else {
             const Class &cl = classes[c];
             // The global class keeps leading columns of A in the shared memory left over.
             const size_t dyn = (!cl.a_shared && !cl.v_shared) ? (smem_cap & ~(size_t)7) : g.smem;
-            cl.fn<<<g.grid, cl.threads, dyn, stream>>>(d_desc + g.first, g.count, d_next + k, req.a, req.a_is_f32,
+            batch_fn(c, g.rows)<<<g.grid, g.threads, dyn, stream>>>(d_desc + g.first, g.count, d_next + k, req.a, req.a_is_f32,
                                                        req.eps, req.max_sweeps, req.sigma, req.v, req.u,
                                                        d_sweeps + g.first, d_ws + gws_base[k], g.gws,
                                                        (int)(dyn / sizeof(double)));

@@ -66,19 +66,21 @@ __host__ __device__ __forceinline__ double rot_q(double c, double s, double x, d
 // and its slot is skipped.  The one definition used by every kernel that
 // derives its pairs instead of reading a table, and by the host-side check
 // (jsvd_round_robin_schedule).
+// (No division: every remainder is of a number within one L of its range.)
 __host__ __device__ __forceinline__ int2 round_robin_pair(int n, int r, int k)
 {
     const int ne = n + (n & 1);
     const int L = ne - 1;
     int i = k;
     if (n & 1) {
-        const int j = 1 + ((n - 1 + r) % L);
+        const int v = n - 1 + r;  // < 2 L
+        const int j = 1 + (v >= L ? v - L : v);
         const int slot = j < ne / 2 ? j : ne - 1 - j;
         if (i >= slot) i += 1;
     }
-    const int i2 = ne - 1 - i;
-    const int p = i == 0 ? 0 : 1 + ((i - 1 - r) % L + L) % L;
-    const int q = 1 + ((i2 - 1 - r) % L + L) % L;
+    const int vp = i - 1 - r, vq = ne - 2 - i - r;  // > -L, < L
+    const int p = i == 0 ? 0 : 1 + (vp < 0 ? vp + L : vp);
+    const int q = 1 + (vq < 0 ? vq + L : vq);
     return make_int2(p, q);
 }
 
