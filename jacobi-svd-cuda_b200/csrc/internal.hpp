@@ -139,3 +139,29 @@ void pc_release_thread_plans();
         if (jsvd_status_ != cudaSuccess)                                             \
             return ::jsvd::cuda_failure(jsvd_status_, #EXPR, __FILE__, __LINE__);    \
     } while (0)
+
+namespace jsvd {
+
+// Launches a kernel that may begin while the previous kernel of the stream ends
+// (programmatic stream serialisation): its launch and its prologue overlap that
+// kernel's tail.  The kernel calls pdl_wait() before it touches global memory,
+// and reads what the previous kernel wrote by loads that do not take the
+// non-coherent path (that one may see lines cached before the wait).
+template <class... Params, class... Args>
+int launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = block;
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    JSVD_CUDA_TRY(cudaLaunchKernelEx(&lc, kernel, static_cast<Params>(args)...));
+    return JSVD_OK;
+}
+
+}  // namespace jsvd

@@ -116,6 +116,9 @@ __global__ void __launch_bounds__(kGramTcThreads)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
+    pdl_launch_dependents();
+    pdl_wait();
+    fence_proxy_async();  // the previous kernel's stores, before TMA reads them
 
     if (warp == 4) {
         if (lane == 0) {
@@ -249,7 +252,10 @@ __global__ void __launch_bounds__(kRotTcThreads)
               const int *__restrict__ flags, int *__restrict__ status)
 {
     const int pair = blockIdx.y;
-    if (flags[pair] == 0) return;  // W = I: the tile stays as it is
+    pdl_launch_dependents();
+    pdl_wait();
+    if (__ldcg(flags + pair) == 0) return;  // W = I: the tile stays as it is
+    fence_proxy_async();  // the previous kernels' stores, before TMA reads them
     extern __shared__ uint8_t smraw[];
     uint8_t *sm = align1024(smraw);
     uint64_t *full = reinterpret_cast<uint64_t *>(sm + kRotBarOff);
@@ -379,6 +385,8 @@ __global__ void __launch_bounds__(kGram64Threads)
     const int nst = (r1 - r0 + kGram64Rows - 1) / kGram64Rows;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int fr = lane >> 2, fk = lane & 3;
+    pdl_launch_dependents();
+    pdl_wait();
     auto issue = [&](int st) {
         double *s = dsm + (st % kGram64Stages) * kW * kGram64LD;
         const int rb = r0 + st * kGram64Rows;
@@ -454,7 +462,9 @@ __global__ void __launch_bounds__(kRot64Threads)
                const double *__restrict__ W, const int *__restrict__ flags)
 {
     const int pair = blockIdx.y;
-    if (flags[pair] == 0) return;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (__ldcg(flags + pair) == 0) return;
     extern __shared__ double dsm[];
     double *Pt = dsm;                   // [64 cols][136]
     double *Ws = dsm + kW * kRot64PLD;  // [64 cols][68]
@@ -752,6 +762,8 @@ __global__ void __launch_bounds__(kEvdThreads, 1)
         s_rounds = 0;
     }
     if (tid <= kEvdMaxInner) sweep_any[tid] = 0;
+    pdl_launch_dependents();
+    pdl_wait();
     // the input Gram, summed over the splits (eight in flight), to buffer 0 in
     // slot coordinates.  A unit is rows 2j, 2j+1 of column c, 2j <= c; columns i
     // and 63 - i have 33 together
@@ -769,7 +781,7 @@ __global__ void __launch_bounds__(kEvdThreads, 1)
             const double *p = part + (size_t)pair * splits * (kW * kW) + ucol[i] * kW + urow[i];
 #pragma unroll 8
             for (int s = 0; s < splits; ++s) {
-                const double2 v = __ldg(reinterpret_cast<const double2 *>(p + (size_t)s * (kW * kW)));
+                const double2 v = __ldcg(reinterpret_cast<const double2 *>(p + (size_t)s * (kW * kW)));
                 acc[i][0] += v.x;
                 acc[i][1] += v.y;
             }
@@ -1441,47 +1453,55 @@ int run_sweep(Work &w, bool tc, double tau, int inner, int sort, cudaStream_t st
     JSVD_CUDA_TRY(cudaMemsetAsync(w.stats, 0, 2 * sizeof(unsigned long long), st));
     const int sample_round[2] = {0, w.rounds / 2};
     const int nsample = w.rounds > 2 ? 2 : 1;
+    const dim3 gram_grid(tc ? w.tc_splits : w.f64_splits, w.npairs), rot_grid(w.x_tiles + w.v_tiles, w.npairs);
+    double *const part = static_cast<double *>(w.part);
+    int last = -1;  // the last sampled round
     for (int r = 0; r < w.rounds; ++r) {
         int si = -1;
         for (int i = 0; i < nsample; ++i)
             if (r == sample_round[i]) si = i;
+        if (si >= 0) last = r;
+        // Each kernel begins while the one before it ends, except where events
+        // or copies stand between them, and except the FP64 Gram, whose early
+        // CTAs slowed the rotation they waited for.  (4096 x 1024, per solve:
+        // tensor-core sweeps 7.67 -> 7.00 ms, FP64 sweeps 7.83 -> 7.30; with the
+        // FP64 Gram 8.15.)
+        const bool overlap = si < 0 && r != last + 1;
+        auto go = [&](bool early, auto kernel, dim3 grid, int threads, size_t smem, auto... args) -> int {
+            if (early) return launch_overlapped(kernel, grid, dim3(threads), smem, st, args...);
+            kernel<<<grid, threads, smem, st>>>(args...);
+            return JSVD_OK;
+        };
         if (si >= 0) cudaEventRecord(w.tev[si][0], st);
-        if (tc) {
-            mx_gram_tc<<<dim3(w.tc_splits, w.npairs), kGramTcThreads, kGramTcSmem, st>>>(
-                w.mxh, w.mxl, w.nb, r, w.tc_chunks, w.tc_chunks_per_split, static_cast<double *>(w.part), w.status);
-            if (si >= 0) {
-                cudaEventRecord(w.tev[si][1], st);
-                cudaMemcpyAsync(w.stats + 4 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
-            }
-            mx_evd<<<w.npairs, kEvdThreads, kEvdSmem, st>>>(static_cast<const double *>(w.part), w.tc_splits, tau, inner,
-                                                            w.nb, r, sort, w.cols, w.W, w.wimg, w.flags, w.stats);
-            if (si >= 0) {
-                cudaMemcpyAsync(w.stats + 5 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
-                cudaEventRecord(w.tev[si][2], st);
-            }
-            mx_rot_tc<<<dim3(w.x_tiles + w.v_tiles, w.npairs), kRotTcThreads, kRotTcSmem, st>>>(
-                w.rxh, w.rxl, w.rvh, w.rvl, w.xh, w.xl, w.rows_pad, w.x_tiles, w.vh, w.vl, w.cols_pad, w.nb, r, w.wimg,
-                w.flags, w.status);
-            ms.tc_gram += 1;
-            ms.tc_rot += 1;
-        } else {
-            mx_gram_f64<<<dim3(w.f64_splits, w.npairs), kGram64Threads, kGram64Smem, st>>>(
-                w.xr, w.rows_pad, w.nb, r, w.f64_rows_per_split, w.rows_pad, static_cast<double *>(w.part));
-            if (si >= 0) {
-                cudaEventRecord(w.tev[si][1], st);
-                cudaMemcpyAsync(w.stats + 4 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
-            }
-            mx_evd<<<w.npairs, kEvdThreads, kEvdSmem, st>>>(static_cast<const double *>(w.part), w.f64_splits, tau, inner,
-                                                            w.nb, r, sort, w.cols, w.W, nullptr, w.flags, w.stats);
-            if (si >= 0) {
-                cudaMemcpyAsync(w.stats + 5 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
-                cudaEventRecord(w.tev[si][2], st);
-            }
-            mx_rot_f64<<<dim3(w.x_tiles + w.v_tiles, w.npairs), kRot64Threads, kRot64Smem, st>>>(
-                w.xr, w.rows_pad, w.x_tiles, w.v64, w.cols_pad, w.nb, r, w.W, w.flags);
-            ms.f64_gram += 1;
-            ms.f64_rot += 1;
+        int rc;
+        if (tc)
+            rc = go(overlap, mx_gram_tc, gram_grid, kGramTcThreads, kGramTcSmem, w.mxh, w.mxl, w.nb, r, w.tc_chunks,
+                    w.tc_chunks_per_split, part, w.status);
+        else
+            rc = go(false, mx_gram_f64, gram_grid, kGram64Threads, kGram64Smem, (const double *)w.xr, (long)w.rows_pad, w.nb, r,
+                    w.f64_rows_per_split, w.rows_pad, part);
+        if (rc != JSVD_OK) return rc;
+        if (si >= 0) {
+            cudaEventRecord(w.tev[si][1], st);
+            cudaMemcpyAsync(w.stats + 4 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
         }
+        rc = go(overlap, mx_evd, dim3(w.npairs), kEvdThreads, kEvdSmem, (const double *)part, (int)gram_grid.x, tau, inner, w.nb,
+                r, sort, w.cols, w.W, tc ? w.wimg : nullptr, w.flags, w.stats);
+        if (rc != JSVD_OK) return rc;
+        if (si >= 0) {
+            cudaMemcpyAsync(w.stats + 5 + 2 * si, w.stats + 1, 8, cudaMemcpyDeviceToDevice, st);
+            cudaEventRecord(w.tev[si][2], st);
+        }
+        if (tc)
+            rc = go(overlap, mx_rot_tc, rot_grid, kRotTcThreads, kRotTcSmem, w.rxh, w.rxl, w.rvh, w.rvl, w.xh, w.xl,
+                    (long)w.rows_pad, w.x_tiles, w.vh, w.vl, (long)w.cols_pad, w.nb, r, (const float *)w.wimg,
+                    (const int *)w.flags, w.status);
+        else
+            rc = go(overlap, mx_rot_f64, rot_grid, kRot64Threads, kRot64Smem, w.xr, (long)w.rows_pad, w.x_tiles, w.v64,
+                    (long)w.cols_pad, w.nb, r, (const double *)w.W, (const int *)w.flags);
+        if (rc != JSVD_OK) return rc;
+        (tc ? ms.tc_gram : ms.f64_gram) += 1;
+        (tc ? ms.tc_rot : ms.f64_rot) += 1;
         if (si >= 0) cudaEventRecord(w.tev[si][3], st);
         ms.evd += 1;
     }

@@ -122,6 +122,9 @@ __device__ __forceinline__ void tma_prefetch_desc(const void *tensor_map)
 
 // Generic-proxy shared-memory writes -> visible to the async proxy (tcgen05.mma
 // operand reads).
+// Orders generic-proxy accesses before async-proxy ones (TMA, bulk copies), of
+// every state space or of shared memory only.
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem()
 {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
