@@ -3,12 +3,19 @@
 // tcgen05 has no FP64 kind, so the FP64 products of this library (CholeskyQR
 // Grams and triangular updates, re-orthogonalisation, U = Q U_x, V = Q1 V_x)
 // run on mma.sync m8n8k4 f64 (DMMA).  Each warp owns a 32 x 32 tile of C (16
-// DMMA tiles, 32 accumulators per lane); a CTA owns BM x BN; operand tiles of
-// BK = 16 are staged in shared memory through a 3-stage cp.async ring.
+// DMMA tiles, 32 accumulators per lane); a CTA of 4 warps owns 64 x 64, two
+// CTAs to an SM, so that one's loads, barriers and epilogue pass under the
+// other's DMMA.  Measured against one 128 x 128 CTA of 16 warps (B200): 4096^3
+// op T,N 4.42 ms, 31.1 TFLOP/s (4.93, 27.9); 1024 x 8192 x 1024 op N,T 0.590
+// ms (0.778); 8192 x 4032 x 64 with beta = 1 0.242 (0.283).  128 x 64 lies
+// between (4.70, 0.692, 0.239).  Three CTAs of 64 x 64, at 168 registers, are
+// 3 % faster still at 4096^3 but 20 % slower where they leave a short second
+// wave (2048^2 lower, k = 4096: 0.65 -> 0.80 ms); four spill.  Operand tiles of BK =
+// 16 are staged in shared memory through a 3-stage cp.async ring.
 // Every operand is stored in shared memory along the dimension that is
 // contiguous in global memory, so global reads are coalesced and shared-memory
 // writes conflict-free:
-//   MN-contiguous [k][mn] (row length BM + 8: fragment reads of 8 x 4 doubles
+//   MN-contiguous [k][mn] (row length 64 + 8: fragment reads of 8 x 4 doubles
 //     take the minimum two wavefronts) for op(A) = N and op(B) = T;
 //   K-contiguous  [mn][k] (row length BK + 4, same property) for op(A) = T and
 //     op(B) = N.
@@ -25,6 +32,8 @@
 namespace jsvd {
 namespace {
 
+constexpr int kBM = 64, kBN = 64;  // tile of C per CTA
+constexpr int kThreads = (kBM / 32) * (kBN / 32) * 32;
 constexpr int kBK = 16;
 constexpr int kStages = 3;
 
@@ -39,13 +48,13 @@ struct OperandTile {
 // Loads the kBK-deep slice k0 of op(X) rows [mn0, mn0 + BMN) into s.  X is
 // column-major with leading dimension ldx.  For op = N of A (and op = T of B)
 // the contiguous global dimension is mn; otherwise it is k.
-template <bool KCONTIG, int BMN, int NT>
+template <bool KCONTIG, int BMN>
 __device__ __forceinline__ void load_tile(double *s, const double *X, long ldx, int mn0, int k0, int MN, int K)
 {
     using Tl = OperandTile<KCONTIG, BMN>;
     constexpr int TOTAL = BMN * kBK;
 #pragma unroll
-    for (int e0 = 0; e0 < TOTAL; e0 += NT) {
+    for (int e0 = 0; e0 < TOTAL; e0 += kThreads) {
         const int e = e0 + (int)threadIdx.x;
         int mn, k;
         if (KCONTIG) {
@@ -67,31 +76,30 @@ __device__ __forceinline__ void load_tile(double *s, const double *X, long ldx, 
     }
 }
 
-template <int BM, int BN, bool TA, bool TB>
-__global__ void __launch_bounds__((BM / 32) * (BN / 32) * 32)
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(kThreads, 2)
     dgemm_kernel(int m, int n, int k, double alpha, const double *__restrict__ A, long lda,
                  const double *__restrict__ B, long ldb, double beta, double *__restrict__ C, long ldc, int lower)
 {
-    constexpr int WN = BN / 32;
-    constexpr int NT = (BM / 32) * WN * 32;
+    constexpr int WN = kBN / 32;
     // op(A) = N: A(m x k) contiguous along m -> MN-contiguous; op(A) = T: K-contiguous.
     // op(B) = N: B(k x n) contiguous along k -> K-contiguous;  op(B) = T: MN-contiguous.
     constexpr bool AK = TA, BKc = !TB;
-    using TA_ = OperandTile<AK, BM>;
-    using TB_ = OperandTile<BKc, BN>;
+    using TA_ = OperandTile<AK, kBM>;
+    using TB_ = OperandTile<BKc, kBN>;
     extern __shared__ double dsm[];
     double *sa = dsm;
     double *sb = dsm + kStages * TA_::ELEMS;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    if (lower && n0 > m0 + BM - 1) return;  // tile strictly above the diagonal
+    const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
+    if (lower && n0 > m0 + kBM - 1) return;  // tile strictly above the diagonal
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = warp / WN, wn = warp % WN;
     const int ktiles = (k + kBK - 1) / kBK;
 
     auto issue = [&](int kt) {
         const int s = kt % kStages;
-        load_tile<AK, BM, NT>(sa + s * TA_::ELEMS, A, lda, m0, kt * kBK, m, k);
-        load_tile<BKc, BN, NT>(sb + s * TB_::ELEMS, B, ldb, n0, kt * kBK, n, k);
+        load_tile<AK, kBM>(sa + s * TA_::ELEMS, A, lda, m0, kt * kBK, m, k);
+        load_tile<BKc, kBN>(sb + s * TB_::ELEMS, B, ldb, n0, kt * kBK, n, k);
     };
 
     double acc[4][4][2];
@@ -131,68 +139,50 @@ __global__ void __launch_bounds__((BM / 32) * (BN / 32) * 32)
     // store to the same array, so one element at a time the epilogue was a chain
     // of 32 loads (a 64 x 64 x 64 product with beta = 1: 20 us, with beta = 0:
     // 7.6 us, alone on the device).
-    // The 128-row tile has registers for half of them at a time.
-    constexpr int kHold = BM >= 128 ? 2 : 4;
+    double old[4][4][2];
+    if (beta != 0.0) {
 #pragma unroll
-    for (int i0 = 0; i0 < 4; i0 += kHold) {
-        double old[kHold][4][2];
-        if (beta != 0.0) {
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int i = 0; i < kHold; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int row = m0 + wm * 32 + (i0 + i) * 8 + fr, col = n0 + wn * 32 + j * 8 + 2 * fk + h;
-                        const bool live = row < m && col < n && !(lower && col > row);
-                        old[i][j][h] = live ? C[(size_t)row + (size_t)col * ldc] : 0.0;
-                    }
-        }
-#pragma unroll
-        for (int i = 0; i < kHold; ++i) {
-            const int row = m0 + wm * 32 + (i0 + i) * 8 + fr;
-            if (row >= m) continue;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int col = n0 + wn * 32 + j * 8 + 2 * fk + h;
-                    if (col >= n || (lower && col > row)) continue;
-                    const double v = alpha * acc[i0 + i][j][h];
-                    C[(size_t)row + (size_t)col * ldc] = (beta == 0.0) ? v : fma(beta, old[i][j][h], v);
+                    const int row = m0 + wm * 32 + i * 8 + fr, col = n0 + wn * 32 + j * 8 + 2 * fk + h;
+                    const bool live = row < m && col < n && !(lower && col > row);
+                    old[i][j][h] = live ? C[(size_t)row + (size_t)col * ldc] : 0.0;
                 }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int row = m0 + wm * 32 + i * 8 + fr;
+        if (row >= m) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int col = n0 + wn * 32 + j * 8 + 2 * fk + h;
+                if (col >= n || (lower && col > row)) continue;
+                const double v = alpha * acc[i][j][h];
+                C[(size_t)row + (size_t)col * ldc] = (beta == 0.0) ? v : fma(beta, old[i][j][h], v);
             }
         }
     }
 }
 
-template <int BM, int BN, bool TA, bool TB>
+template <bool TA, bool TB>
 int launch(cudaStream_t st, int m, int n, int k, double alpha, const double *A, long lda, const double *B, long ldb,
            double beta, double *C, long ldc, int lower)
 {
-    constexpr int NT = (BM / 32) * (BN / 32) * 32;
     constexpr size_t smem = sizeof(double) * kStages *
-                            (OperandTile<TA, BM>::ELEMS + OperandTile<!TB, BN>::ELEMS);
+                            (OperandTile<TA, kBM>::ELEMS + OperandTile<!TB, kBN>::ELEMS);
     static_assert(smem <= 227 * 1024, "dgemm tile does not fit shared memory");
-    auto kern = dgemm_kernel<BM, BN, TA, TB>;
+    auto kern = dgemm_kernel<TA, TB>;
     if (smem > 48 * 1024)
         JSVD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const dim3 grid((m + BM - 1) / BM, (n + BN - 1) / BN);
-    kern<<<grid, NT, smem, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
+    const dim3 grid((m + kBM - 1) / kBM, (n + kBN - 1) / kBN);
+    kern<<<grid, kThreads, smem, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
     JSVD_CUDA_TRY(cudaGetLastError());
     return JSVD_OK;
-}
-
-template <bool TA, bool TB>
-int dispatch(cudaStream_t st, int m, int n, int k, double alpha, const double *A, long lda, const double *B,
-             long ldb, double beta, double *C, long ldc, int lower)
-{
-    // Large outputs: 128 x 128 tiles (16 warps); otherwise 64 x 64 (4 warps) so
-    // that a GEMM of a 1024-column factor still fills the 148 SMs.
-    const long tiles128 = (long)((m + 127) / 128) * ((n + 127) / 128);
-    if (tiles128 >= 2 * 148)
-        return launch<128, 128, TA, TB>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
-    return launch<64, 64, TA, TB>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
 }
 
 thread_local unsigned long long t_launches = 0;
@@ -209,10 +199,10 @@ int dgemm(cudaStream_t st, char opA, char opB, int m, int n, int k, double alpha
     if (m > 65535 * 64 || n > 65535 * 64) return invalid_argument("dgemm: matrix too large for the tile grid.");
     ++t_launches;
     const bool ta = (opA == 'T' || opA == 't'), tb = (opB == 'T' || opB == 't');
-    if (!ta && !tb) return dispatch<false, false>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
-    if (!ta && tb) return dispatch<false, true>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
-    if (ta && !tb) return dispatch<true, false>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
-    return dispatch<true, true>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
+    if (!ta && !tb) return launch<false, false>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
+    if (!ta && tb) return launch<false, true>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
+    if (ta && !tb) return launch<true, false>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
+    return launch<true, true>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
 }
 
 }  // namespace jsvd
