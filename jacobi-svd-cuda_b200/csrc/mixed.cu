@@ -1556,7 +1556,9 @@ int orthogonalise(Work &w, cudaStream_t st, int steps, double *residual)
     const int n = w.cols_pad;
     const size_t nn = (size_t)n * n;
     for (int i = 0; i < steps; ++i) {
-        if (int rc = dgemm(st, 'T', 'N', n, n, n, 1.0, w.v64, n, w.v64, n, 0.0, w.e64, n); rc != JSVD_OK) return rc;
+        if (int rc = dgemm(st, 'T', 'N', n, n, n, 1.0, w.v64, n, w.v64, n, 0.0, w.e64, n, kGemmSymmetric);
+            rc != JSVD_OK)
+            return rc;
         JSVD_CUDA_TRY(cudaMemsetAsync(w.stats + 2, 0, sizeof(unsigned long long), st));
         mx_minus_identity_max<<<grid_for(nn), 256, 0, st>>>(w.e64, n, w.stats + 2);
         JSVD_CUDA_TRY(cudaGetLastError());

@@ -1204,7 +1204,8 @@ int PlainPlan::gram_converged(cudaStream_t st, bool &converged)
         JSVD_CUDA_TRY(cudaMallocHost((void **)&h_gram_count, sizeof(unsigned)));
         JSVD_CUDA_TRY(cudaStreamSynchronize(stream));
     }
-    if (const int rc = dgemm(st, 'T', 'N', (int)n, (int)n, (int)m, 1.0, a_cur, lda, a_cur, lda, 0.0, gram, (long)n, 1);
+    if (const int rc = dgemm(st, 'T', 'N', (int)n, (int)n, (int)m, 1.0, a_cur, lda, a_cur, lda, 0.0, gram, (long)n,
+                             kGemmLower);
         rc != JSVD_OK)
         return rc;
     JSVD_CUDA_TRY(cudaMemsetAsync(gram_count, 0, sizeof(unsigned), st));

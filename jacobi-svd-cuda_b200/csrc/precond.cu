@@ -308,7 +308,7 @@ __global__ void pc_lower_to_upper(const double *__restrict__ L, double *__restri
 int chol_qr_pass(cudaStream_t st, double *Q, double *Qout, int m, int n, double *G, double *Lm, double *Linv,
                  double *R, bool shift, int *d_status)
 {
-    JSVD_GEMM_TRY(dgemm(st, 'T', 'N', n, n, m, 1.0, Q, m, Q, m, 0.0, G, n, 1));
+    JSVD_GEMM_TRY(dgemm(st, 'T', 'N', n, n, m, 1.0, Q, m, Q, m, 0.0, G, n, kGemmLower));
     if (shift) {
         pc_shift_diagonal<<<1, 256, 0, st>>>(G, n, m);
         JSVD_CUDA_TRY(cudaGetLastError());
@@ -325,7 +325,8 @@ int chol_qr_pass(cudaStream_t st, double *Q, double *Qout, int m, int n, double 
                                 Lm + (size_t)k0 * n + k0 + kb, n));
             // G22 -= L21 L21^T (lower)
             JSVD_GEMM_TRY(dgemm(st, 'N', 'T', rest, rest, kb, -1.0, Lm + (size_t)k0 * n + k0 + kb, n,
-                                Lm + (size_t)k0 * n + k0 + kb, n, 1.0, G + (size_t)(k0 + kb) * n + k0 + kb, n, 1));
+                                Lm + (size_t)k0 * n + k0 + kb, n, 1.0, G + (size_t)(k0 + kb) * n + k0 + kb, n,
+                                kGemmLower));
         }
     }
     for (int j0 = 0, blk = 0; j0 < n; j0 += kNb, ++blk) {
@@ -493,8 +494,8 @@ int precond_impl(const double *d_a, size_t rows, size_t cols, const jsvd_config 
         if (r == JSVD_OK) r = chol_qr_pass(s2, Xb, Xa, rows, n, G, Lm, Linv, Rb, false, d_status);
         if (r == JSVD_OK) r = chol_qr_pass(s2, Xa, Xb, rows, n, G, Lm, Linv, Rc, false, d_status);
         if (r != JSVD_OK) return r;
-        JSVD_GEMM_TRY(dgemm(s2, 'N', 'N', n, n, n, 1.0, Rb, n, Ra, n, 0.0, Tm, n));
-        JSVD_GEMM_TRY(dgemm(s2, 'N', 'N', n, n, n, 1.0, Rc, n, Tm, n, 0.0, Ra, n));
+        JSVD_GEMM_TRY(dgemm(s2, 'N', 'N', n, n, n, 1.0, Rb, n, Ra, n, 0.0, Tm, n, kGemmUpper));
+        JSVD_GEMM_TRY(dgemm(s2, 'N', 'N', n, n, n, 1.0, Rc, n, Tm, n, 0.0, Ra, n, kGemmUpper));
         return JSVD_OK;
     };
     // Runs a QR stage: directly, or (a plan on its second use onwards) as a
