@@ -19,6 +19,7 @@
 //     take the minimum two wavefronts) for op(A) = N and op(B) = T;
 //   K-contiguous  [mn][k] (row length BK + 4, same property) for op(A) = T and
 //     op(B) = N.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,6 +32,8 @@
 
 namespace jsvd {
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int kBM = 64, kBN = 64;  // tile of C per CTA
 constexpr int kThreads = (kBM / 32) * (kBN / 32) * 32;
@@ -93,15 +96,20 @@ __global__ void __launch_bounds__(kThreads, 2)
     double *sa = dsm;
     double *sb = dsm + kStages * TA_::ELEMS;
     const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
-    if ((kForm == kGemmSymmetric || lower) && n0 > m0 + kBM - 1) return;  // tile strictly above the diagonal
+    constexpr bool kSplit = kForm == kGemmGram;
+    if ((kForm == kGemmSymmetric || kSplit || lower) && n0 > m0 + kBM - 1) return;  // tile strictly above the diagonal
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = warp / WN, wn = warp % WN;
     // Upper times upper: k in [m0, n0 + kBN), empty below the diagonal; the
     // terms left out are products with a zero.  1/6 of the full product's work.
     // With V^T V from its lower tiles, a mixed solve of 8192 x 4096: 425 -> 405
     // ms, of 1777 x 611: 12.83 -> 12.58 ms.
-    const int first = kForm == kGemmUpper ? m0 / kBK : 0;
-    const int last = ((kForm == kGemmUpper ? min(k, n0 + kBN) : k) + kBK - 1) / kBK;
+    int first = kForm == kGemmUpper ? m0 / kBK : 0;
+    int last = ((kForm == kGemmUpper ? min(k, n0 + kBN) : k) + kBK - 1) / kBK;
+    if constexpr (kSplit) {
+        first = (int)((long)last * blockIdx.z / gridDim.z);
+        last = (int)((long)last * (blockIdx.z + 1) / gridDim.z);
+    }
 
     auto issue = [&](int kt) {
         const int s = kt % kStages;
@@ -142,6 +150,33 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
     }
     cp_async_wait<0>();
+    if constexpr (kSplit) {
+        // The cluster's CTAs hold parts of one tile: each leaves its part in
+        // shared memory, then adds an equal share of the tile's columns over the
+        // ranks, in their order.
+        constexpr int kLd = kBM + 2;
+        static_assert(kBN * kLd <= kStages * (TA_::ELEMS + TB_::ELEMS), "the part fits the staging buffers");
+        cg::cluster_group cluster = cg::this_cluster();
+        const int parts = (int)gridDim.z;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    dsm[(wn * 32 + j * 8 + 2 * fk + h) * kLd + wm * 32 + i * 8 + fr] = acc[i][j][h];
+        cluster.sync();
+        const int share = kBN / parts;
+        for (int e = (int)threadIdx.x; e < share * kBM; e += kThreads) {
+            const int c = (int)blockIdx.z * share + e / kBM, r = e % kBM;
+            double sum = 0.0;
+            for (int p = 0; p < parts; ++p) sum += cluster.map_shared_rank(dsm, p)[c * kLd + r];
+            if (m0 + r < m && n0 + c < n && n0 + c <= m0 + r) C[(size_t)(m0 + r) + (size_t)(n0 + c) * ldc] = alpha * sum;
+        }
+        cluster.sync();  // no CTA leaves while another reads its part
+        return;
+    }
     // C's old values are all loaded before any store: a load cannot pass a
     // store to the same array, so one element at a time the epilogue was a chain
     // of 32 loads (a 64 x 64 x 64 product with beta = 1: 20 us, with beta = 0:
@@ -177,6 +212,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
 }
 
+// lower: for kGemmGram the number of parts, else whether only the lower
+// triangle is written
 template <bool TA, bool TB, GemmForm kForm>
 int launch(cudaStream_t st, int m, int n, int k, double alpha, const double *A, long lda, const double *B, long ldb,
            double beta, double *C, long ldc, int lower)
@@ -188,9 +225,37 @@ int launch(cudaStream_t st, int m, int n, int k, double alpha, const double *A, 
     if (smem > 48 * 1024)
         JSVD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const dim3 grid((m + kBM - 1) / kBM, (n + kBN - 1) / kBN);
+    if constexpr (kForm == kGemmGram) {
+        cudaLaunchAttribute attr = {};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim = {1, 1, (unsigned)lower};
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid.x, grid.y, (unsigned)lower);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        JSVD_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, 1));
+        return JSVD_OK;
+    }
     kern<<<grid, kThreads, smem, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower);
     JSVD_CUDA_TRY(cudaGetLastError());
     return JSVD_OK;
+}
+
+// Parts of the sum over k of an n x n Gram: as many (a power of two, at most 8)
+// as keep the tiles on and below the diagonal within two CTAs to an SM, each
+// part at least 128 deep: unsplit, the 36 tiles of a 512-column Gram leave 112
+// SMs idle and one warp per scheduler with nothing to hide its loads.  B200,
+// QR-preconditioned solve of 2048 x 512 10.80 -> 10.53 ms, mixed 1777 x 611
+// 12.58 -> 12.32.  The parts' shorter sums round less than the single one.
+int gram_parts(int n, int k)
+{
+    const long t = (n + kBN - 1) / kBN, tiles = t * (t + 1) / 2;
+    int parts = 1;
+    while (parts < 8 && tiles * parts * 2 <= 2 * 148 && k / (parts * 2) >= 128) parts *= 2;
+    return parts;
 }
 
 thread_local unsigned long long t_launches = 0;
@@ -207,6 +272,14 @@ int dgemm(cudaStream_t st, char opA, char opB, int m, int n, int k, double alpha
     if (m > 65535 * 64 || n > 65535 * 64) return invalid_argument("dgemm: matrix too large for the tile grid.");
     ++t_launches;
     const bool ta = (opA == 'T' || opA == 't'), tb = (opB == 'T' || opB == 't');
+    if (form == kGemmGram) {
+        if (!ta || tb || m != n || beta != 0.0)
+            return invalid_argument("dgemm: the product does not have the form asked for.");
+        const int parts = gram_parts(n, k);
+        if (parts > 1)
+            return launch<true, false, kGemmGram>(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, parts);
+        form = kGemmLower;
+    }
     const auto run = [&](auto of) { return of(st, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, form == kGemmLower); };
     if (form == kGemmSymmetric || form == kGemmUpper) {
         const bool upper = form == kGemmUpper;

@@ -18,6 +18,9 @@ enum GemmForm : int {
     // A and B are upper triangular, ops N and N: tiles below the diagonal are zero,
     // and a tile (i, j) sums k from i to j only.  m = n = k and beta = 0.
     kGemmUpper = 3,
+    // kGemmLower of ops T and N with beta = 0 whose sum over k may be split in
+    // up to 8 parts (by shape only), added in a fixed order
+    kGemmGram = 4,
 };
 
 // C = alpha op(A) op(B) + beta C, column-major, op = 'N' or 'T'.  op(A) is

@@ -308,7 +308,7 @@ __global__ void pc_lower_to_upper(const double *__restrict__ L, double *__restri
 int chol_qr_pass(cudaStream_t st, double *Q, double *Qout, int m, int n, double *G, double *Lm, double *Linv,
                  double *R, bool shift, int *d_status)
 {
-    JSVD_GEMM_TRY(dgemm(st, 'T', 'N', n, n, m, 1.0, Q, m, Q, m, 0.0, G, n, kGemmLower));
+    JSVD_GEMM_TRY(dgemm(st, 'T', 'N', n, n, m, 1.0, Q, m, Q, m, 0.0, G, n, kGemmGram));
     if (shift) {
         pc_shift_diagonal<<<1, 256, 0, st>>>(G, n, m);
         JSVD_CUDA_TRY(cudaGetLastError());
