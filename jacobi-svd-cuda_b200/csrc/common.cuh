@@ -109,12 +109,6 @@ __device__ __forceinline__ void group_barrier(int id, int threads)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// Arrives at that barrier without waiting.
-__device__ __forceinline__ void group_barrier_arrive(int id, int threads)
-{
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 // 1 / d to about one ulp for 2^-1000 <= d < 2^1000 (reciprocal_in_range), from
 // the hardware's approximation r (relative error e = 1 - d r of about 2^-20) as
 // r (1 + e + e^2).
