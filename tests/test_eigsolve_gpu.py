@@ -49,3 +49,22 @@ def test_scaled_rotations():
     finally:
         jsvd.mixed_set_options(None)
     check(a, r, scale)
+
+
+def test_small_rotations_keep_unit_columns():
+    """Columns orthogonal to about 1e-12: every pair rotates once, by angles below
+    1e-8, whose cosine rounds to 1.  V's leading entries are then 1 to within
+    2 ulp (products by 1 and sums of terms below 1e-16); a cosine that is one ulp
+    off to one side would move them by about n ulp."""
+    m, n = 300, 256
+    a = np.zeros((m, n))
+    a[np.arange(n), np.arange(n)] = np.linspace(2.0, 1.0, n)
+    a += 1e-12 * np.random.default_rng(9).standard_normal((m, n))
+    jsvd.mixed_set_options(precondition=0, tc_max_sweeps=0)
+    try:
+        r = jsvd.mixed_svd(a, jsvd.default_config(epsilon=1e-14))
+    finally:
+        jsvd.mixed_set_options(None)
+    lead = np.abs(r.v).max(axis=0)
+    assert np.abs(r.v).max() > 0 and np.count_nonzero(r.v) > n  # it rotated
+    assert np.abs(lead - 1.0).max() <= 4.5e-16
