@@ -237,7 +237,7 @@ __device__ __forceinline__ void sweep_rounds(ColA colA, double *V, int m, int n,
         // phase 2: angles, one thread per pair
         for (int k = threadIdx.x; k < npairs; k += blockDim.x) {
             double c, s;
-            if (rotation_params(st_pp[k], st_qq[k], st_pq[k], eps, c, s)) s_rot = 1;
+            if (rotation_params_flat(st_pp[k], st_qq[k], st_pq[k], eps, c, s)) s_rot = 1;
             st_cs[k] = make_double2(c, s);
         }
         __syncthreads();
@@ -620,7 +620,7 @@ __device__ __forceinline__ bool warp_angle_cl(const double *x, const double *y, 
     // Far below the threshold (by a factor of two, well above the rounding of
     // either side) nothing rotates: most pairs of the last sweeps stop here.
     if (pq * pq < (0.25 * eps * eps) * (fmax(pp, 0.0) * fmax(qq, 0.0))) return false;
-    return rotation_params(pp, qq, pq, eps, c, s);
+    return rotation_params_flat(pp, qq, pq, eps, c, s);
 }
 
 // A CTA's share of a member: its slots [k0, k0 + S) of the circle's half, and

@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kFusedMaxThreads, 1)
                     qq += __shfl_xor_sync(0xffffffffu, qq, off);
                     pq += __shfl_xor_sync(0xffffffffu, pq, off);
                 }
-                rotation_params(pp, qq, pq, eps, c, s);
+                rotation_params_flat(pp, qq, pq, eps, c, s);
             };
             ++x;
             ++dummy;
