@@ -155,6 +155,14 @@ void jsvd_plain_stats_get(jsvd_plain_stats *out);
 void jsvd_plain_set_sweep_mode(int mode);
 int jsvd_plain_get_sweep_mode(void);
 
+/* How a plan of this shape launches a sweep: *form 0 = one kernel per round, 1 =
+ * *rounds rounds per launch with *slots pair slots per CTA, 2 = one persistent
+ * kernel.  threads as in jsvd_config; sms: the device's SMs; cooperative: whether
+ * the persistent kernel can be launched on it.  The outputs may be NULL.  No CUDA
+ * call. */
+int jsvd_plain_sweep_form(size_t rows, size_t columns, int threads, int mode, int sms, int cooperative, int *form,
+                          int *rounds, int *slots);
+
 /* Forces (1) or releases (0) the in-place global-memory form of the plain
  * path's deferred V pass for plans created afterwards.  That form is used by
  * itself for more than 25600 columns, where a row of V does not fit a CTA's

@@ -170,9 +170,10 @@ int acquire_plain_plan(size_t m, size_t n, int T, double eps, cudaStream_t strea
     int dev = 0;
     JSVD_CUDA_TRY(cudaGetDevice(&dev));
     auto &plans = thread_cache().plans;
+    const int mode = sweep_mode();  // read once: another thread may set it meanwhile
     for (size_t i = 0; i < plans.size(); ++i) {
         PlainPlan *p = plans[i].get();
-        if (p->device == dev && p->m == m && p->n == n && p->T == T && p->eps == eps && p->mode == sweep_mode() &&
+        if (p->device == dev && p->m == m && p->n == n && p->T == T && p->eps == eps && p->mode == mode &&
             p->vpass_global_forced == vpass_global_forced()) {
             std::rotate(plans.begin() + i, plans.begin() + i + 1, plans.end());
             *out = plans.back().get();
@@ -185,11 +186,8 @@ int acquire_plain_plan(size_t m, size_t n, int T, double eps, cudaStream_t strea
     if (own == nullptr) return cuda_failure(cudaGetLastError(), "cudaStreamCreateWithFlags", __FILE__, __LINE__);
     if (own != stream) JSVD_CUDA_TRY(cudaStreamSynchronize(stream));
     std::unique_ptr<PlainPlan> plan;
-    int rc = PlainPlan::create(dev, m, n, T, eps, own, plan);
+    int rc = PlainPlan::create(dev, m, n, T, eps, mode, own, plan);
     if (rc != JSVD_OK) return rc;
-    plan->mode = sweep_mode();
-    plan->use_pdl = plan->mode == 2;
-    plan->angle_once = plan->mode != 3;
     plans.push_back(std::move(plan));
     size_t total = 0;
     for (auto &p : plans) total += p->bytes;

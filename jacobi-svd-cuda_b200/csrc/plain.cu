@@ -995,7 +995,24 @@ PlainPlan::~PlainPlan()
     if (prev >= 0) cudaSetDevice(prev);
 }
 
-int PlainPlan::create(int dev, size_t m_, size_t n_, int T_, double eps_, cudaStream_t stream,
+SweepForm sweep_form(int mode, size_t m, size_t n, int T, int sms, bool cooperative)
+{
+    SweepForm f;
+    if (n < 2) return f;
+    if (mode == 1 && cooperative) {
+        f.kind = SweepForm::kPersistent;
+    } else if (mode == 0 && T == kFusedT) {
+        const FusedShape fs = fused_shape((int)m, (int)n, sms);
+        if (fs.rounds > 0 && pick_fused((int)m).threads * (fs.slots + fs.rounds - 1) <= kFusedMaxThreads) {
+            f.kind = SweepForm::kFused;
+            f.rounds = fs.rounds;
+            f.slots = fs.slots;
+        }
+    }
+    return f;
+}
+
+int PlainPlan::create(int dev, size_t m_, size_t n_, int T_, double eps_, int mode_, cudaStream_t stream,
                       std::unique_ptr<PlainPlan> &out)
 {
     auto plan = std::make_unique<PlainPlan>();
@@ -1005,6 +1022,9 @@ int PlainPlan::create(int dev, size_t m_, size_t n_, int T_, double eps_, cudaSt
     plan->n = n_;
     plan->T = T_;
     plan->eps = eps_;
+    plan->mode = mode_;
+    plan->use_pdl = mode_ == 2;
+    plan->angle_once = mode_ != 3;
     plan->lda = (long)m_;
     plan->ldv = (long)n_;
     std::vector<int2> host_pairs;
@@ -1058,18 +1078,17 @@ int PlainPlan::create(int dev, size_t m_, size_t n_, int T_, double eps_, cudaSt
         SweepFn sfn = pick_sweep(T_, (int)m_);
         JSVD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sfn, T_, 0));
         const int half = (int)((n_ + (n_ & 1)) / 2);
-        if (coop && per_sm > 0 && sweep_mode() == 1) {
+        const SweepForm form = sweep_form(mode_, m_, n_, T_, sms, coop && per_sm > 0);
+        if (form.kind == SweepForm::kPersistent) {
             const int max_ctas = per_sm * sms;
             plan->slots_per_cta = (half + max_ctas - 1) / max_ctas;
             plan->sweep_grid = (half + plan->slots_per_cta - 1) / plan->slots_per_cta;
             JSVD_CUDA_TRY(cudaMallocAsync((void **)&plan->flags, sizeof(int) * (plan->sweep_grid + 1), stream));
             plan->persistent = true;
         }
-        const FusedShape fs = fused_shape((int)m_, (int)n_, sms);
-        if (fs.rounds > 0 && T_ == kFusedT && sweep_mode() == 0 &&
-            pick_fused((int)m_).threads * (fs.slots + fs.rounds - 1) <= kFusedMaxThreads) {
-            plan->fused_rounds = fs.rounds;
-            plan->fused_slots = fs.slots;
+        if (form.kind == SweepForm::kFused) {
+            plan->fused_rounds = form.rounds;
+            plan->fused_slots = form.slots;
             JSVD_CUDA_TRY(cudaMallocAsync((void **)&plan->a_w2, sizeof(double) * m_ * n_, stream));
             // the same cap for every plan, like the V pass's above
             JSVD_CUDA_TRY(cudaFuncSetAttribute(pick_fused((int)m_).fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1417,6 +1436,23 @@ extern "C" int jsvd_test_wait_limit(int which, int limit_ms, int preset, int *de
                                                  ").");
             return JSVD_ERR_RUNTIME;
         }
+        return JSVD_OK;
+    });
+}
+
+extern "C" int jsvd_plain_sweep_form(size_t rows, size_t columns, int threads, int mode, int sms, int cooperative,
+                                     int *form, int *rounds, int *slots)
+{
+    return c_entry([&]() -> int {
+        set_last_error(JSVD_OK, "");
+        if (rows < columns || columns == 0 || dims_out_of_range(rows, columns))
+            return invalid_argument("rows >= columns >= 1 within the supported range.");
+        if (mode < 0 || mode > 3) return invalid_argument("mode must be in [0, 3].");
+        if (sms < 1) return invalid_argument("sms must be positive.");
+        const SweepForm f = sweep_form(mode, rows, columns, reduction_lanes(threads), sms, cooperative != 0);
+        if (form) *form = f.kind;
+        if (rounds) *rounds = f.rounds;
+        if (slots) *slots = f.slots;
         return JSVD_OK;
     });
 }

@@ -23,6 +23,21 @@ constexpr size_t kVpassSmemCap = 200 * 1024;
 bool vpass_global_forced();
 void set_vpass_global_forced(bool on);
 
+// How a plan launches a sweep.  One kind, so that no plan can hold buffers of two
+// forms: a fused plan's A alternates between two copies, a persistent sweep
+// rotates one in place.
+struct SweepForm {
+    enum Kind { kRounds = 0, kFused = 1, kPersistent = 2 };
+    Kind kind = kRounds;
+    int rounds = 0, slots = 0;  // kFused: rounds per launch, pair slots per CTA
+};
+
+// The form of an m x n plan of `mode` (see sweep_mode) with T reduction lanes on
+// a device of `sms` SMs; `cooperative`: the persistent kernel can be launched.
+// A function of its arguments: the process-wide mode may change at any time, so
+// it is read once per plan and passed in.
+SweepForm sweep_form(int mode, size_t m, size_t n, int T, int sms, bool cooperative);
+
 struct PlainPlan {
     int device = -1;
     cudaStream_t stream = nullptr;  // allocation / release stream (the creating thread's)
@@ -52,7 +67,7 @@ struct PlainPlan {
     int sweep_launches() const { return fused_rounds > 0 ? fused_launches() : rounds; }
     bool persistent = false;      // one cooperative launch per sweep
     int slots_per_cta = 1, sweep_grid = 0;
-    int mode = 0;         // sweep_mode() at creation
+    int mode = 0;         // the sweep mode it was created for
     bool use_pdl = false;     // programmatic dependent launch between rounds
     bool angle_once = false;  // rounds reduce and derive the angle in one warp
     unsigned long long uses = 0;
@@ -77,7 +92,7 @@ struct PlainPlan {
     PlainPlan(const PlainPlan &) = delete;
     PlainPlan &operator=(const PlainPlan &) = delete;
 
-    static int create(int dev, size_t m, size_t n, int T, double eps, cudaStream_t stream,
+    static int create(int dev, size_t m, size_t n, int T, double eps, int mode, cudaStream_t stream,
                       std::unique_ptr<PlainPlan> &out);
     int ensure_host_staging();
     int enqueue_rounds(cudaStream_t st, int parity);

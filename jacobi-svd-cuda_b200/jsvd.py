@@ -199,7 +199,7 @@ def exported_symbols() -> list[str]:
         "jsvd_mixed_options_default", "jsvd_mixed_set_options", "jsvd_mixed_svd", "jsvd_mixed_svd_device",
         "jsvd_mixed_stats_get", "jsvd_mixed_stats_reset", "jsvd_dgemm_device", "jsvd_mixed_test_round",
         "jsvd_test_wait_limit", "jsvd_mixed_builtin_tuning",
-        "jsvd_mixed_sweep_history", "jsvd_batch_set_cluster_classes",
+        "jsvd_mixed_sweep_history", "jsvd_batch_set_cluster_classes", "jsvd_plain_sweep_form",
     ]
 
 
@@ -278,6 +278,8 @@ def lib() -> ctypes.CDLL:
         L.jsvd_plain_set_sweep_mode.argtypes = [I]
         L.jsvd_plain_set_sweep_mode.restype = None
         L.jsvd_plain_get_sweep_mode.restype = I
+        L.jsvd_plain_sweep_form.argtypes = [S, S, I, I, I, I] + [ctypes.POINTER(I)] * 3
+        L.jsvd_plain_sweep_form.restype = I
         L.jsvd_blockpair_svd_device.argtypes = [P, S, S, ctypes.POINTER(Config), P, P, P, P, P]
         L.jsvd_blockpair_svd_device.restype = I
         L.jsvd_blockpair_svd.argtypes = [P, S, S, ctypes.POINTER(Config), P, P, P, P]
@@ -602,6 +604,15 @@ def set_sweep_mode(mode: int) -> None:
     (default), 1 = persistent sweep, 2 = as 0 with programmatic dependent
     launch, 3 = as 0 with every warp deriving the angle."""
     lib().jsvd_plain_set_sweep_mode(mode)
+
+
+def plain_sweep_form(m: int, n: int, threads: int = 256, mode: int = 0, sms: int = 148,
+                     cooperative: bool = True) -> tuple[int, int, int]:
+    """(form, rounds per launch, slots per CTA) of a plan of this shape: form 0 one
+    kernel per round, 1 several rounds per launch, 2 one persistent kernel."""
+    out = [ctypes.c_int(0) for _ in range(3)]
+    check(lib().jsvd_plain_sweep_form(m, n, threads, mode, sms, int(cooperative), *map(ctypes.byref, out)))
+    return tuple(x.value for x in out)
 
 
 def plain_stats() -> PlainStats:
