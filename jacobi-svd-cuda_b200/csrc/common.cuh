@@ -109,19 +109,47 @@ __device__ __forceinline__ void group_barrier(int id, int threads)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// 1 / d to about one ulp for 2^-1000 <= d < 2^1000 (reciprocal_in_range), from
-// the hardware's approximation r (relative error e = 1 - d r of about 2^-20) as
-// r (1 + e + e^2).
+// 1 / d and 1 / sqrt(a) from the hardware's approximations, each by one step of
+// third order.  PTX documents rcp.approx.ftz.f64 and rsqrt.approx.ftz.f64 to take
+// the argument's and to give the result's upper 32 bits: about 2^-20 relative,
+// and a result r of at most 21 significant bits.
+//   1 / d:       e = 1 - d r,      1 / d = r / (1 - e)             = r (1 + e + e^2 + ...)
+//   1 / sqrt(a): e = 1 - a r^2,    1 / sqrt(a) = r (1 - e)^(-1/2)  = r (1 + e/2 + 3 e^2/8 + ...)
+// (the geometric and the binomial series: the hyperpower iteration of order
+// three, Altman 1960, and Householder's, 1970).  r^2 has at most 42 bits and is
+// exact, so e is the exact residual rounded once, and the result is within half
+// an ulp and the terms left out (e^3 and 5 e^3 / 16, under 0.1 ulp for |e| <=
+// 2^-19), to no side: with a r rounded before the second product, the result
+// near a = 1 was off by its last bit, mostly to one side.
+__device__ __forceinline__ double hw_reciprocal(double d)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    return r;
+}
+__device__ __forceinline__ double hw_rsqrt(double a)
+{
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
+    return r;
+}
+// For 2^-1000 <= d < 2^1000 (reciprocal_in_range).
 __device__ __forceinline__ bool reciprocal_in_range(double d)
 {
     return (unsigned)__double2hiint(d) - 0x01700000u < 0x7e700000u - 0x01700000u;
 }
 __device__ __forceinline__ double approx_reciprocal(double d)
 {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double r = hw_reciprocal(d);
     const double e = fma(-d, r, 1.0);
     return fma(r, fma(e, e, e), r);
+}
+// For a normal a in [2^-1000, 2^1000).
+__device__ __forceinline__ double approx_rsqrt(double a)
+{
+    const double r = hw_rsqrt(a);
+    const double e = fma(-a, r * r, 1.0);
+    return fma(r * e, fma(e, 0.375, 0.5), r);
 }
 
 // Rutishauser rotation for the 2x2 Gram [pp pq; pq qq]; returns true when the

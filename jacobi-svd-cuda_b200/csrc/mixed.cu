@@ -615,16 +615,6 @@ constexpr EvdBlocks evd_make_blocks()
 }
 __device__ const EvdBlocks kEvdBlocks = evd_make_blocks();
 
-// 1 / sqrt(a) to about one ulp for a normal a: one third-order step on the
-// hardware's approximation y (e = 1 - a y^2): y (1 + e / 2 + 3 e^2 / 8).
-__device__ __forceinline__ double approx_rsqrt(double a)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    const double e = fma(-(a * y), y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // Rotation of [pp pq; pq qq] that annihilates pq, with the reference's
 // threshold test (|pq| > tau sqrt(pp qq), squared, and |pq| > 1e-300).
 //   t = tan(theta), the smaller root of t^2 + 2 zeta t - 1 = 0 with
@@ -657,9 +647,10 @@ __device__ __forceinline__ bool evd_rotation(double pp, double qq, double tau2, 
     const double hs = (0.5 * ae) * rho;  // sin 2theta / 2
     const double rc = approx_rsqrt(c2);  // 1 / c
     const double c1 = c2 * rc, sa = hs * rc, ta = sa * rc;
-    // c from c^2 + s^2 = 1, to rounding.  The approximation's last bit errs to
-    // one side near c = 1, and every rotation would scale its columns by it:
-    // ||V^T V - I|| of a 4096 x 1024 solve 2.3e-13 with it, 1.1e-12 without.
+    // c from c^2 + s^2 = 1, to rounding: an error of c that many small rotations
+    // share scales their columns.  With a reciprocal square root whose last bit
+    // erred to one side near 1, ||V^T V - I|| of a 4096 x 1024 solve was 2.3e-13
+    // with this line and 1.1e-12 without; with approx_rsqrt and the line 2.3e-13.
     const double ca = fma(0.5 * fma(-sa, sa, fma(-c1, c1, 1.0)), rc, c1);
     const double thr = tau2 * (fmax(pp, 0.0) * fmax(qq, 0.0));
     const bool rot = fabs(pq) > 1.0e-300 && pq * pq > thr;
