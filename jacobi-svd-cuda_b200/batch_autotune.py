@@ -79,9 +79,9 @@ def render_table(report: dict, meta: dict, cluster: dict) -> str:
     lines += [
         " *",
         " * CTAs per matrix: the classes whose bit is set in JSVD_BATCH_CLUSTER_CLASSES",
-        " * are solved by a thread-block cluster per matrix (2, 4 or 8 CTAs, the",
-        " * smallest that holds it), the others by one CTA per matrix; a class goes",
-        " * over only when that is more than 2% faster.",
+        " * are solved by a thread-block cluster per matrix (2, 4 or 8 CTAs; class 3",
+        " * only while its members are few), the others by one CTA per matrix; a class",
+        " * goes over only when that is more than 2% faster.",
         f" * {cluster['note']}",
         " * class: ms one CTA per matrix, ms clusters -> chosen",
     ]

@@ -16,13 +16,13 @@
  * distribution, class 2 over 2000; classes 3 and 4 as generated)
  *
  * CTAs per matrix: the classes whose bit is set in JSVD_BATCH_CLUSTER_CLASSES
- * are solved by a thread-block cluster per matrix (2, 4 or 8 CTAs), the others
- * by one CTA per matrix; a class goes over only when that is more than 2%
- * faster.
+ * are solved by a thread-block cluster per matrix (2, 4 or 8 CTAs; class 3
+ * only while its members are few), the others by one CTA per matrix; a class
+ * goes over only when that is more than 2% faster.
  * Timed on NVIDIA B200 (148 SMs), 2026-12-05, over 2000 FP32-stored matrices (m ~ U{16..256}, n ~ U{8..m}), all classes, mean of 3 runs.
  * class: ms one CTA per matrix, ms clusters -> chosen
  *   2: 17.6, 22.7 -> one CTA
- *   3: 25.3, 33.0 -> one CTA
+ *   3: 25.3 -> clusters while few
  *   4: 119.5, 95.7 -> clusters
  */
 #pragma once
@@ -30,4 +30,4 @@
 #define JSVD_BATCH_TUNING_TABLE \
     { {128, 4, 0}, {256, 2, 0}, {512, 1, 0}, {512, 1, 0}, {512, 1, 0} }
 
-#define JSVD_BATCH_CLUSTER_CLASSES 0x10
+#define JSVD_BATCH_CLUSTER_CLASSES 0x18

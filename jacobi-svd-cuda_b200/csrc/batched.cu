@@ -9,10 +9,10 @@
 //   class 3  : A in shared memory, V in a per-CTA slice of global memory
 //   class 4  : A and V in global memory (L2-resident per-CTA slices), the
 //              leading columns of A that fit in shared memory kept there
-// By default the members of class 4 are instead solved by a thread-block
-// cluster each (batch_cluster_kernel: A and V in the cluster's distributed
-// shared memory; see the section "cluster classes"); a member no cluster holds
-// stays with its class's kernel.
+// By default the members of class 4, and of class 3 while they are few, are
+// instead solved by a thread-block cluster each (batch_cluster_kernel: A and V in
+// the cluster's distributed shared memory; see the section "cluster classes"); a
+// member no cluster holds stays with its class's kernel.
 // Launch shapes per class (threads, CTAs per SM, grid cap) come from the
 // compiled-in table batch_tuning_table.h, which batch_autotune.py writes from
 // jsvd_batch_autotune (defined at the end of this file).
@@ -470,8 +470,8 @@ __global__ void __launch_bounds__(256) batch_finish_kernel(const StepDesc *__res
 // What bounds it (B200, 228 x 189 members on 8 CTAs of 12 slots): one member
 // alone takes 2.9 us per round, a chain of dot products (0.5 us), angle (0.5),
 // rotation (0.8, at the shared-memory port's rate) and the cluster barrier; two
-// members on the same SMs take 3.0 us for both.  So a cluster is chosen such
-// that two of its CTAs share an SM where the member allows it.  Registers decide
+// members on the same SMs take 3.0 us for both.  So many members share SMs by
+// two where their shape allows it (cluster_choice).  Registers decide
 // the rest: at two CTAs per SM a thread has 80, and with the member's shape and
 // the ring indices of every buffer kept in them the loops' own values went to
 // local memory (5.2 us per round; in shared memory now, ClusterRound).  100
@@ -884,33 +884,101 @@ ClusterFn cluster_fn(int C, bool tall, bool share)
     return share ? cluster_fn_c<false, true>(C) : cluster_fn_c<false, false>(C);
 }
 
-// Size classes whose members go to clusters where one fits (bit c = class c;
-// classes 2-4 only), initially the compiled-in tuning table's choice.
-// Process-wide.
+// Size classes whose members may go to clusters (bit c = class c; classes 2-4
+// only; class 3 while its members are few: cluster_choice), initially the
+// compiled-in tuning table's choice.  Process-wide.
 #ifndef JSVD_BATCH_CLUSTER_CLASSES
-#define JSVD_BATCH_CLUSTER_CLASSES (1 << 4)
+#define JSVD_BATCH_CLUSTER_CLASSES (1 << 3 | 1 << 4)
 #endif
 std::atomic<int> g_cluster_mask{JSVD_BATCH_CLUSTER_CLASSES};  // the tuning table's choice
 int batch_cluster_mask() { return g_cluster_mask.load(std::memory_order_relaxed); }
 
-// Cluster of an m x n member: the smallest (2, 4, 8 CTAs) in which two CTAs
-// share an SM's memory with at most one pair slot per warp (share), so that
-// one member's loads and stores run beside the other's arithmetic; else the
-// smallest that holds the member with an SM per CTA; 0 when none does.  At
-// least two slots per CTA.
-int cluster_size_for(int m, int n, size_t smem_cap, bool &share)
+// Cluster of a member; C = 0: the class's one-CTA kernel.  share: two CTAs to an
+// SM, so that one member's loads and stores run beside the other's arithmetic.
+struct ClusterChoice {
+    int C = 0;
+    bool share = false;
+};
+
+// Clusters that the device holds at once: own[i] of 2 << i CTAs with an SM each,
+// shared4 of four CTAs at two to an SM.
+struct ClusterCapacity {
+    int sms = 0, own[3] = {}, shared4 = 0;
+};
+
+// The cluster of an m x n member of class `cls` that has `members` in the batch.
+// The larger the cluster, the sooner its member is done and the fewer run side by
+// side, so the choice goes by how many have to.  ms for 14, 32, 70 and 592 equal
+// members (B200):
+//                        500 x 80 (class 4)   250 x 140 (class 4)   350 x 70 (class 3)
+//   8 CTAs, an SM each   1.5  4.4  7.3  58    2.7  7.9   13  104    1.2  3.5  5.8  46
+//   8 CTAs, shared       1.8  2.2  6.3  38    2.7  3.5  9.7   62    1.4  1.6  4.6  28
+//   4 CTAs, an SM each   1.8  1.8  5.1  30    4.7  4.7   14   83    1.4  1.4  4.0  23
+//   4 CTAs, shared       2.1  2.1  2.8  23    does not fit          1.6  1.6  2.5  16
+//   2 CTAs, an SM each   3.1  3.1  3.1  24    does not fit          2.5  2.5  2.5  19
+//   the class's kernel   7.7  7.7  7.7  31     13   13   14   54    4.1  4.1  4.1  16
+// While all are resident at once: the largest cluster with an SM per CTA, before
+// that eight shared CTAs where they keep the warps busy (9 to 12 slots on 12
+// warps).  More members: in class 4 two CTAs where they hold the member, four
+// shared ones where those keep the warps busy, else eight shared ones or the
+// smallest that holds it.  In class 3 whichever takes less, by whole waves: a wave
+// of the class's kernel lasts 1.5 to 1.6 waves of two CTAs (more than 256 rows:
+// 1.7 to 2.2), 2.4 of four.
+ClusterChoice cluster_choice(int m, int n, int cls, long members, size_t smem_cap, const ClusterCapacity &cap)
 {
     const int half = (n + (n & 1)) / 2;
-    share = true;
-    for (int C : {2, 4, 8})
-        if (half >= 2 * C && cluster_slots_max(n, C) <= kClusterThreadsShared / 32 &&
-            cluster_smem_bytes(m, n, C) <= smem_cap / 2 - 1024)
-            return C;
-    share = false;
-    for (int C : {2, 4, 8})
-        if (half >= 2 * C && cluster_slots_max(n, C) <= kClusterMaxSlots && cluster_smem_bytes(m, n, C) <= smem_cap)
-            return C;
-    return 0;
+    auto own = [&](int C) {  // at least two slots per CTA
+        return half >= 2 * C && cluster_slots_max(n, C) <= kClusterMaxSlots && cluster_smem_bytes(m, n, C) <= smem_cap;
+    };
+    auto shared = [&](int C, int least) {
+        const int slots = cluster_slots_max(n, C);
+        return half >= 2 * C && slots >= least && slots <= kClusterThreadsShared / 32 &&
+               cluster_smem_bytes(m, n, C) <= smem_cap / 2 - 1024;
+    };
+    auto waves = [&](int at_once) { return (members + at_once - 1) / std::max(at_once, 1); };
+    if (own(8) && members <= cap.own[2]) return {8, false};
+    if (shared(8, 9) && 8 * members <= 2 * cap.sms) return {8, true};
+    if (own(4) && members <= cap.own[1]) return {4, false};
+    const int C = own(2) ? 2 : (own(4) ? 4 : (own(8) ? 8 : 0));
+    if (cls == 3) {
+        const int tenths = C == 2 ? (m > kLanes ? 17 : 15) : (C == 4 ? 24 : 40);
+        return C > 0 && 10 * waves(cap.own[C / 4]) <= tenths * waves(cap.sms) ? ClusterChoice{C, false} : ClusterChoice{};
+    }
+    if (C == 2) {
+        if (shared(4, 9) && (members <= cap.shared4 || members > cap.own[0])) return {4, true};
+        return {2, false};
+    }
+    // (8 slots: 512 x 128 7.3 ms against 8.0 for 37 members, 76 against 72 for 592)
+    if (shared(8, 2 * members <= cap.sms ? 8 : 9)) return {8, true};
+    return {C, false};
+}
+
+int cluster_capacity(int dev, int sms, size_t smem_cap, ClusterCapacity &cap)
+{
+    static std::atomic<int> known[64][4];
+    cap.sms = sms;
+    for (int i = 0; i < 4; ++i) {
+        int &out = i < 3 ? cap.own[i] : cap.shared4;
+        out = dev >= 0 && dev < 64 ? known[dev][i].load(std::memory_order_relaxed) : 0;
+        if (out > 0) continue;
+        const int C = i < 3 ? 2 << i : 4;
+        const ClusterFn fn = cluster_fn(C, false, i == 3);
+        JSVD_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)C;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3((unsigned)C);
+        lc.blockDim = dim3(i == 3 ? kClusterThreadsShared : kClusterThreads);
+        lc.dynamicSmemBytes = i == 3 ? smem_cap / 2 - 1024 : smem_cap;
+        lc.attrs = at;
+        lc.numAttrs = 1;
+        JSVD_CUDA_TRY(cudaOccupancyMaxActiveClusters(&out, fn, &lc));
+        if (dev >= 0 && dev < 64) known[dev][i].store(out, std::memory_order_relaxed);
+    }
+    return JSVD_OK;
 }
 
 using BatchFn = void (*)(const BatchDesc *, int, int *, const void *, int, double, int, double *, double *,
@@ -1094,6 +1162,9 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
     };
     auto work = [&](int i) { return member_work(all[i].m, all[i].n); };
     const int mask = batch_cluster_mask();
+    ClusterCapacity capacity;
+    if (mask != 0)
+        if (const int rc = cluster_capacity(dev, sms, smem_cap, capacity); rc != JSVD_OK) return rc;
     std::vector<Group> groups;
     std::vector<BatchDesc> ordered;
     ordered.reserve(count);
@@ -1104,11 +1175,14 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
         // by kernel: own (0-2, by rows), clusters of 2, 4, 8 (3-5), + 3 sharing an
         // SM, + 6 tall
         std::vector<int> sub[15];
+        // (a launch shape given for class 3 is its own kernel's)
+        const bool on = (mask >> c) & 1 && !(c == 3 && req.tuning != nullptr && req.tuning[3].threads > 0);
         for (int i : members[c]) {
-            bool share = false;
-            const int C = ((mask >> c) & 1) ? cluster_size_for(all[i].m, all[i].n, smem_cap, share) : 0;
+            ClusterChoice cc;
+            if (on) cc = cluster_choice(all[i].m, all[i].n, c, (long)members[c].size(), smem_cap, capacity);
             const BatchRows rows = c <= 2 ? batch_rows(all[i].m) : std::min(batch_rows(all[i].m), kRows256);
-            sub[C == 0 ? (int)rows : (C == 2 ? 3 : (C == 4 ? 4 : 5)) + (share ? 3 : 0) + (all[i].m > kLanes ? 6 : 0)]
+            sub[cc.C == 0 ? (int)rows
+                          : (cc.C == 2 ? 3 : (cc.C == 4 ? 4 : 5)) + (cc.share ? 3 : 0) + (all[i].m > kLanes ? 6 : 0)]
                 .push_back(i);
         }
         for (int s : {14, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 0, 1, 2}) {

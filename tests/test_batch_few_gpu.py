@@ -1,0 +1,59 @@
+"""Which kernel a member of the two largest size classes gets: by its shape and
+by how many members of its class the batch has (csrc/batched.cu:
+cluster_choice).  The counts stand on both sides of every line of that rule on
+a device of 148 SMs; the results are the plain path's bytes whatever is chosen,
+and a few members of class 3 are not left to one CTA each.
+"""
+import time
+
+import numpy as np
+import pytest
+
+import jsvd
+import workloads
+
+pytestmark = pytest.mark.gpu
+
+# class 3: with C = 2, without; class 4: two and four CTAs, eight shared, eight
+# slots, more than 12 slots, none but eight
+SHAPES = [(350, 70), (165, 160), (500, 80), (250, 140), (512, 128), (256, 200), (256, 256)]
+
+
+@pytest.mark.parametrize("count", [1, 13, 17, 32, 36, 40, 70, 74, 80, 160])
+@pytest.mark.parametrize("m,n", SHAPES)
+def test_bytes_for_every_choice(cuda_device, m, n, count):
+    cfg = jsvd.default_config(epsilon=1e-12, max_sweeps=1)
+    a = workloads.gaussian_splitmix(m, n, seed=m + n)
+    w = jsvd.plain_svd(a, cfg)
+    b = jsvd.DeviceBatch([a] * count, cuda_device, want_u=True)
+    b.solve(cfg)
+    for u, s, v, sw in b.results():
+        assert sw == w.sweeps
+        assert np.array_equal(s, w.sigma) and np.array_equal(u, w.u) and np.array_equal(v, w.v)
+
+
+def _best_ms(b, cfg, reps=5):
+    import torch
+
+    best = np.inf
+    for _ in range(reps):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        b.solve(cfg)
+        best = min(best, time.perf_counter() - t)
+    return best * 1e3
+
+
+@pytest.mark.parametrize("m,n", [(350, 70), (200, 130)])
+def test_few_members_of_class_3_are_spread_over_the_device(cuda_device, m, n):
+    """Eight members on 148 SMs: by clusters 0.25 and 0.35 of the time of one CTA
+    each; half is allowed."""
+    cfg = jsvd.default_config(epsilon=1e-12)
+    b = jsvd.DeviceBatch([workloads.gaussian_splitmix(m, n, seed=i) for i in range(8)], cuda_device)
+    chosen = _best_ms(b, cfg)
+    old = jsvd.batch_set_cluster_classes(0)
+    try:
+        alone = _best_ms(b, cfg)
+    finally:
+        jsvd.batch_set_cluster_classes(old)
+    assert chosen <= 0.5 * alone
