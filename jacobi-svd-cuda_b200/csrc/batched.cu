@@ -288,6 +288,16 @@ __device__ __forceinline__ bool batch_sweep(ColA colA, double *V, int m, int n, 
     return any;
 }
 
+// The launches of a class do not depend on each other, and each begins when the
+// CTAs of the one before have begun, on the SMs that it leaves idle.  The end of
+// such a launch: it is not complete before that one is, so that what follows it
+// in the stream finds both done.  (One thread waits; the other CTAs give their
+// SMs back.)
+__device__ __forceinline__ void end_after_previous()
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) pdl_wait();
+}
+
 template <bool kAShared, bool kVShared, BatchRows kRows>
 __global__ void __launch_bounds__(512) batch_kernel(const BatchDesc *__restrict__ descs, int count,
                                                     int *__restrict__ next, const void *__restrict__ a_all,
@@ -306,11 +316,12 @@ __global__ void __launch_bounds__(512) batch_kernel(const BatchDesc *__restrict_
     __shared__ int s_rot;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     double *gws = workspace + (size_t)blockIdx.x * ws_stride;
+    pdl_launch_dependents();
     for (;;) {
         if (threadIdx.x == 0) s_idx = atomicAdd(next, 1);
         __syncthreads();
         const int idx = s_idx;
-        if (idx >= count) return;
+        if (idx >= count) return end_after_previous();
         const BatchDesc d = descs[idx];
         const int m = d.m, n = d.n;
         const int half = round_half(n);
@@ -717,6 +728,7 @@ __global__ void __launch_bounds__(kShare ? kClusterThreadsShared : kClusterThrea
         s_rot = 0;
         s_stamp = 0;
     }
+    pdl_launch_dependents();
     for (;;) {
         int ld, mp, m, rounds, S, jt0, bot_base;
         {
@@ -727,7 +739,7 @@ __global__ void __launch_bounds__(kShare ? kClusterThreadsShared : kClusterThrea
             // every CTA has read the index and finished the previous member's
             // outputs before any CTA writes into another's buffers or exits
             cluster.sync();
-            if (idx >= count) return;
+            if (idx >= count) return end_after_previous();
             const BatchDesc d = read_desc(descs, idx);
             const ClusterShare sh(d.m, d.n, rank, C);
             // round 0: position p holds column p; V = I
@@ -1283,22 +1295,29 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
         // The classes run one after another on one stream: persistent CTAs of
         // a class hold their SMs until its queue drains, and concurrent classes
         // starved each other (a 512-thread CTA of the global class fills an
-        // SM's register file).
-        if (k == 0 || groups[k - 1].cls != c) JSVD_CUDA_TRY(cudaEventRecord(ts->c0[c], stream));
+        // SM's register file).  The groups of a class, which are one class split
+        // by kernel, overlap: each begins on the SMs that the one before leaves
+        // (end_after_previous).  One after another, four members of class 2
+        // between 100 and 300 rows took 8.6 ms, the longest alone 3.4.
+        const bool first_of_class = k == 0 || groups[k - 1].cls != c;
+        if (first_of_class) JSVD_CUDA_TRY(cudaEventRecord(ts->c0[c], stream));
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = first_of_class ? 0 : 1;
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3((unsigned)g.grid);
+        lc.stream = stream;
+        lc.attrs = at;
+        lc.numAttrs = 1;
         class_count[c] += g.count;
         if (g.csize > 0) {
-            cudaLaunchConfig_t lc = {};
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = (unsigned)g.csize;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            lc.gridDim = dim3((unsigned)g.grid);
+            at[1].id = cudaLaunchAttributeClusterDimension;
+            at[1].val.clusterDim.x = (unsigned)g.csize;
+            at[1].val.clusterDim.y = 1;
+            at[1].val.clusterDim.z = 1;
+            lc.numAttrs = 2;
             lc.blockDim = dim3(g.share ? kClusterThreadsShared : kClusterThreads);
             lc.dynamicSmemBytes = g.smem;
-            lc.stream = stream;
-            lc.attrs = at;
-            lc.numAttrs = 1;
             JSVD_CUDA_TRY(cudaLaunchKernelEx(&lc, cluster_fn(g.csize, g.tall, g.share), (const BatchDesc *)(d_desc + g.first), g.count,
                                              d_next + k, req.a, req.a_is_f32, req.eps, req.max_sweeps, req.sigma,
                                              req.v, req.u, d_sweeps + g.first));
@@ -1306,11 +1325,12 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
             const Class &cl = classes[c];
             // The global class keeps leading columns of A in the shared memory left over.
             const size_t dyn = (!cl.a_shared && !cl.v_shared) ? (smem_cap & ~(size_t)7) : g.smem;
-            batch_fn(c, g.rows)<<<g.grid, g.threads, dyn, stream>>>(d_desc + g.first, g.count, d_next + k, req.a, req.a_is_f32,
-                                                       req.eps, req.max_sweeps, req.sigma, req.v, req.u,
-                                                       d_sweeps + g.first, d_ws + gws_base[k], g.gws,
-                                                       (int)(dyn / sizeof(double)));
-            JSVD_CUDA_TRY(cudaGetLastError());
+            lc.blockDim = dim3((unsigned)g.threads);
+            lc.dynamicSmemBytes = dyn;
+            JSVD_CUDA_TRY(cudaLaunchKernelEx(&lc, batch_fn(c, g.rows), (const BatchDesc *)(d_desc + g.first), g.count,
+                                             d_next + k, req.a, req.a_is_f32, req.eps, req.max_sweeps, req.sigma,
+                                             req.v, req.u, d_sweeps + g.first, d_ws + gws_base[k], g.gws,
+                                             (int)(dyn / sizeof(double))));
         }
         if (k + 1 == groups.size() || groups[k + 1].cls != c) JSVD_CUDA_TRY(cudaEventRecord(ts->c1[c], stream));
         ++launches;

@@ -57,3 +57,33 @@ def test_few_members_of_class_3_are_spread_over_the_device(cuda_device, m, n):
     finally:
         jsvd.batch_set_cluster_classes(old)
     assert chosen <= 0.5 * alone
+
+
+@pytest.mark.parametrize("shapes", [[(100, 90), (200, 90), (300, 50)], [(200, 130), (350, 70), (165, 160)]])
+def test_groups_of_a_class_overlap(cuda_device, shapes):
+    """Three members of one class for three kernels (class 2 by rows, class 3 by
+    cluster): together they take the longest one's time, and 0.8 of the sum of
+    their times is allowed.  One after another they take the sum."""
+    cfg = jsvd.default_config(epsilon=1e-12)
+    mats = [workloads.gaussian_splitmix(m, n, seed=m + n) for m, n in shapes]
+    together = _best_ms(jsvd.DeviceBatch(mats, cuda_device), cfg)
+    alone = sum(_best_ms(jsvd.DeviceBatch([a], cuda_device), cfg) for a in mats)
+    assert together <= 0.8 * alone
+
+
+@pytest.mark.parametrize("copies", [1, 12])
+def test_bytes_of_overlapping_groups(cuda_device, copies):
+    shapes = [(40, 30), (200, 20), (500, 10), (100, 60), (200, 45), (300, 30), (100, 90), (200, 90), (300, 50),
+              (200, 130), (350, 70), (165, 160), (500, 80), (250, 140), (512, 128), (256, 200)]
+    cfg = jsvd.default_config(epsilon=1e-12, max_sweeps=2)
+    mats = [workloads.gaussian_splitmix(m, n, seed=m + n) for m, n in shapes]
+    want = [jsvd.plain_svd(a, cfg) for a in mats]
+    b = jsvd.DeviceBatch(mats * copies, cuda_device, want_u=True)
+    for _ in range(3):
+        for x in (b.sigma, b.u, b.v):
+            x.fill_(-1.0)
+        b.solve(cfg)
+        for i, (u, s, v, sw) in enumerate(b.results()):
+            w = want[i % len(want)]
+            assert sw == w.sweeps
+            assert np.array_equal(s, w.sigma) and np.array_equal(u, w.u) and np.array_equal(v, w.v)
