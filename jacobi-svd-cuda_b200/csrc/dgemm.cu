@@ -3,15 +3,12 @@
 // tcgen05 has no FP64 kind, so the FP64 products of this library (CholeskyQR
 // Grams and triangular updates, re-orthogonalisation, U = Q U_x, V = Q1 V_x)
 // run on mma.sync m8n8k4 f64 (DMMA).  Each warp owns a 32 x 32 tile of C (16
-// DMMA tiles, 32 accumulators per lane); a CTA of 4 warps owns 64 x 64, two
-// CTAs to an SM, so that one's loads, barriers and epilogue pass under the
-// other's DMMA.  Measured against one 128 x 128 CTA of 16 warps (B200): 4096^3
-// op T,N 4.42 ms, 31.1 TFLOP/s (4.93, 27.9); 1024 x 8192 x 1024 op N,T 0.590
-// ms (0.778); 8192 x 4032 x 64 with beta = 1 0.242 (0.283).  128 x 64 lies
-// between (4.70, 0.692, 0.239).  Three CTAs of 64 x 64, at 168 registers, are
-// 3 % faster still at 4096^3 but 20 % slower where they leave a short second
-// wave (2048^2 lower, k = 4096: 0.65 -> 0.80 ms); four spill.  Operand tiles of BK =
-// 16 are staged in shared memory through a 3-stage cp.async ring.
+// DMMA tiles, 32 accumulators per lane); a CTA of 4 warps owns 64 x 64, two or
+// three CTAs to an SM (three_ctas), so that one's loads, barriers and epilogue
+// pass under the other's DMMA.  Measured against one 128 x 128 CTA of 16 warps
+// (B200): 4096^3 op T,N 4.42 ms, 31.1 TFLOP/s (4.93, 27.9); 1024 x 8192 x 1024 op
+// N,T 0.590 ms (0.778); 128 x 64 lies between (4.70, 0.692).  Operand tiles of
+// BK = 16 are staged in shared memory through a 3-stage cp.async ring.
 // Every operand is stored in shared memory along the dimension that is
 // contiguous in global memory, so global reads are coalesced and shared-memory
 // writes conflict-free:
@@ -23,6 +20,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <type_traits>
 
 #include "dgemm.hpp"
 #include "internal.hpp"
@@ -80,9 +79,11 @@ __device__ __forceinline__ void load_tile(double *s, const double *X, long ldx, 
 }
 
 // kForm: the forms with a triangle have kernels of their own, because their
-// bounds in the general one cost it 6 % (168 registers for 202).
-template <bool TA, bool TB, GemmForm kForm>
-__global__ void __launch_bounds__(kThreads, 2)
+// bounds in the general one cost it 6 % (168 registers for 202).  kBeta: with
+// three CTAs to an SM, whose registers are the tighter ones, beta = 0 has a
+// kernel without C's old values (1 to 2 %); otherwise it is decided at run time.
+template <bool TA, bool TB, GemmForm kForm, int kCtas, bool kBeta>
+__global__ void __launch_bounds__(kThreads, kCtas)
     dgemm_kernel(int m, int n, int k, double alpha, const double *__restrict__ A, long lda,
                  const double *__restrict__ B, long ldb, double beta, double *__restrict__ C, long ldc, int lower)
 {
@@ -182,7 +183,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     // of 32 loads (a 64 x 64 x 64 product with beta = 1: 20 us, with beta = 0:
     // 7.6 us, alone on the device).
     double old[4][4][2];
-    if (beta != 0.0) {
+    const bool add = kCtas == 2 ? beta != 0.0 : kBeta;
+    if (add) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 const int col = n0 + wn * 32 + j * 8 + 2 * fk + h;
                 if (col >= n || (lower && col > row)) continue;
                 const double v = alpha * acc[i][j][h];
-                C[(size_t)row + (size_t)col * ldc] = (beta == 0.0) ? v : fma(beta, old[i][j][h], v);
+                C[(size_t)row + (size_t)col * ldc] = add ? fma(beta, old[i][j][h], v) : v;
                 if (kForm == kGemmSymmetric && n0 < m0) C[(size_t)col + (size_t)row * ldc] = v;
             }
         }
@@ -214,14 +216,14 @@ __global__ void __launch_bounds__(kThreads, 2)
 
 // lower: for kGemmGram the number of parts, else whether only the lower
 // triangle is written
-template <bool TA, bool TB, GemmForm kForm>
+template <bool TA, bool TB, GemmForm kForm, int kCtas = 2, bool kBeta = true>
 int launch(cudaStream_t st, int m, int n, int k, double alpha, const double *A, long lda, const double *B, long ldb,
            double beta, double *C, long ldc, int lower)
 {
     constexpr size_t smem = sizeof(double) * kStages *
                             (OperandTile<TA, kBM>::ELEMS + OperandTile<!TB, kBN>::ELEMS);
     static_assert(smem <= 227 * 1024, "dgemm tile does not fit shared memory");
-    auto kern = dgemm_kernel<TA, TB, kForm>;
+    auto kern = dgemm_kernel<TA, TB, kForm, kCtas, kBeta>;
     if (smem > 48 * 1024)
         JSVD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const dim3 grid((m + kBM - 1) / kBM, (n + kBN - 1) / kBN);
@@ -244,6 +246,32 @@ int launch(cudaStream_t st, int m, int n, int k, double alpha, const double *A, 
     return JSVD_OK;
 }
 
+// SMs of the current device.
+int device_sms()
+{
+    static std::atomic<int> known[64];
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+    if (dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
+}
+
+// Whether a product of `tiles` tiles runs three CTAs to an SM (168 registers) or
+// two (202).  Two take the tiles of an SM in pairs, three in threes, and a short
+// last wave costs nearly a whole one: with the tiles per SM rounded up, 512 x N x
+// 1024 op N,N takes (us, B200, two / three)
+//   1: 76 / 77   2: 99 / 101   3: 182 / 148   4: 183 / 225   5: 265 / 225
+//   6: 265 / 269   7: 348 / 310   8: 348 / 347   9: 431 / 388   28: 1180 / 1150
+// and lower triangles the same way (k = 2048, 300 tiles: 290 / 263, 528: 332 / 410).
+bool three_ctas(long tiles)
+{
+    const int sms = device_sms();
+    const long load = (tiles + sms - 1) / sms;
+    return load >= 8 || load == 3 || load == 5 || load == 7;
+}
+
 // Parts of the sum over k of an n x n Gram: as many (a power of two, at most 8)
 // as keep the tiles on and below the diagonal within two CTAs to an SM, each
 // part at least 128 deep: unsplit, the 36 tiles of a 512-column Gram leave 112
@@ -254,7 +282,7 @@ int gram_parts(int n, int k)
 {
     const long t = (n + kBN - 1) / kBN, tiles = t * (t + 1) / 2;
     int parts = 1;
-    while (parts < 8 && tiles * parts * 2 <= 2 * 148 && k / (parts * 2) >= 128) parts *= 2;
+    while (parts < 8 && tiles * parts * 2 <= 2 * device_sms() && k / (parts * 2) >= 128) parts *= 2;
     return parts;
 }
 
@@ -287,10 +315,17 @@ int dgemm(cudaStream_t st, char opA, char opB, int m, int n, int k, double alpha
             return invalid_argument("dgemm: the product does not have the form asked for.");
         return upper ? run(launch<false, false, kGemmUpper>) : run(launch<true, false, kGemmSymmetric>);
     }
-    if (!ta && !tb) return run(launch<false, false, kGemmFull>);
-    if (!ta && tb) return run(launch<false, true, kGemmFull>);
-    if (ta && !tb) return run(launch<true, false, kGemmFull>);
-    return run(launch<true, true, kGemmFull>);
+    const long mt = (m + kBM - 1) / kBM, nt = (n + kBN - 1) / kBN, diagonal = std::min(mt, nt);
+    const bool three = three_ctas(form == kGemmLower ? diagonal * mt - diagonal * (diagonal - 1) / 2 : mt * nt);
+    const auto pick = [&](auto opa, auto opb) {
+        constexpr bool A_ = decltype(opa)::value, B_ = decltype(opb)::value;
+        if (!three) return run(launch<A_, B_, kGemmFull>);
+        return beta != 0.0 ? run(launch<A_, B_, kGemmFull, 3, true>) : run(launch<A_, B_, kGemmFull, 3, false>);
+    };
+    const std::true_type T{};
+    const std::false_type N{};
+    if (!ta) return tb ? pick(N, T) : pick(N, N);
+    return tb ? pick(T, T) : pick(T, N);
 }
 
 }  // namespace jsvd
