@@ -253,6 +253,16 @@ __device__ __forceinline__ void sweep_rounds(ColA colA, double *V, int m, int n,
     }
 }
 
+// sweep_rounds for any number of rows beside those for few, with registers of its
+// own: sharing theirs it lost 8 % to what the kernel had without them (a 500 x 40
+// request of the serving core).
+template <bool kApart, class ColA>
+__device__ __noinline__ void tall_rounds(ColA colA, double *V, int m, int n, double eps, double *st_pp, double *st_qq,
+                                         double *st_pq, double2 *st_cs, int &s_rot)
+{
+    sweep_rounds<0, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+}
+
 // What a kernel knows about its members' rows: nothing, at most kLanes, at
 // most kLanes / 2, or that they vary (the loops for every bound in one kernel,
 // which costs the longest of them their registers).
@@ -280,7 +290,7 @@ __device__ __forceinline__ bool batch_sweep(ColA colA, double *V, int m, int n, 
         else if (m <= 64) sweep_rounds<2, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
         else if (!kMany || m <= 128) sweep_rounds<4, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
         else if (m <= 256) sweep_rounds<kMany ? 8 : 4, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
-        else sweep_rounds<kMany ? 0 : 4, kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
+        else if constexpr (kMany) tall_rounds<kApart>(colA, V, m, n, eps, st_pp, st_qq, st_pq, st_cs, s_rot);
     }
     const bool any = s_rot != 0;
     __syncthreads();  // every thread has read the flag before it is reset
