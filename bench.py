@@ -820,7 +820,7 @@ def run_batch(args, rank: int, world: int, device):
                                f"log-uniform [1/kappa,1], kappa log-uniform [1e1,1e6] (seed 3); sigma and V",
                    "path": "batched persistent kernels, plain arithmetic: one CTA per matrix for the size classes "
                            "that fit one CTA's shared memory, one thread-block cluster per matrix (A and V in "
-                           "distributed shared memory) for the largest",
+                           "distributed shared memory) for the largest and, while its members are few, the next",
                    "epsilon": 1e-14, "mean_sweeps": float(np.mean(b.sweeps)),
                    "l2": "flushed between steps (256 MiB write)", "parallelism": f"replicas x{world}",
                    "generation_s": gen_s, "step_ms": step_ms,

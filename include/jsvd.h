@@ -142,16 +142,18 @@ typedef struct jsvd_plain_stats {
 
 void jsvd_plain_stats_get(jsvd_plain_stats *out);
 
-/* How the plain path launches a sweep (process-wide, read when a plan is
- * created): 0 = one kernel per round, replayed from a CUDA graph, each CTA
- * reducing its pair's dot products and deriving the angle once, in one warp
+/* How the plain path launches a sweep (process-wide, read once when a plan is
+ * looked up): 0 = several rounds per kernel up to 1024 rows at
+ * threads_per_block 256, each launched while the previous one drains
+ * (programmatic dependent launch), else one kernel per round; replayed from a
+ * CUDA graph, a pair's dot products reduced and its angle derived once
  * (default); 1 = one persistent cooperative kernel per sweep whose CTAs
  * synchronise with their neighbours through per-CTA round counters (bounded
- * waits); 2 = as 0 with programmatic dependent launch, each round scheduled
- * while the previous one drains; 3 = as 0 with every warp reducing and
- * deriving the angle itself (one barrier fewer, eight times the FP64 work).
- * All give bit-identical results.  Measured per 512-row round on B200: mode 0
- * 2.6 us, mode 3 2.9 us, mode 2 3.9 us, mode 1 6.9 us. */
+ * waits); 2 = one kernel per round with programmatic dependent launch; 3 = one
+ * kernel per round, every warp reducing and deriving the angle itself (one
+ * barrier fewer, eight times the FP64 work).  All give bit-identical results.
+ * Measured per round of a 512 x 512 solve on B200: mode 0 1.5 us, mode 2 2.7
+ * us, mode 3 2.9 us, mode 1 7.0 us. */
 void jsvd_plain_set_sweep_mode(int mode);
 int jsvd_plain_get_sweep_mode(void);
 
@@ -199,7 +201,8 @@ int jsvd_residuals(const double *a, const double *u, const double *sigma, const 
                    size_t columns, jsvd_residual_report *out);
 
 /* ---- batched solver ---------------------------------------------------------
- * Many independent matrices in one persistent launch per size class.  The
+ * Many independent matrices in a few persistent launches per size class (one
+ * per bound on the members' rows and per kind of thread-block cluster).  The
  * reference solves them one call at a time from a host thread pool
  * (src/pipeline.cpp:799-807 -> one_sided_jacobi_svd); this replaces that loop
  * for matrices that are all resident on the device.  Arithmetic per matrix is
@@ -333,7 +336,7 @@ typedef struct jsvd_batch_stats {
     unsigned long long sweeps;
     double kernel_ms; /* device time of the persistent launches (events) */
     unsigned long long class_count[5]; /* matrices per size class */
-    double class_ms[5];                /* device time of each class's launch */
+    double class_ms[5];                /* device time of each class's launches */
 } jsvd_batch_stats;
 
 void jsvd_batch_stats_get(jsvd_batch_stats *out);

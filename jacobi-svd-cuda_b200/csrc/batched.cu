@@ -1,8 +1,10 @@
 // Batched one-sided Jacobi SVD: thousands of independent small matrices,
-// one persistent launch per size class, largest class first (sm_100a).
+// persistent launches per size class, largest class first (sm_100a).  A class's
+// members are split by the kernel that suits them: the one-CTA kernel by a bound
+// on their rows, clusters by their size.
 //
 // Each CTA pulls matrix indices from a device work queue (one atomic counter
-// per class; matrices sorted by work, largest first) and solves the whole
+// per launch; matrices sorted by work, largest first) and solves the whole
 // matrix before taking the next one.  Where the FP64 working copies live
 // depends on the class:
 //   class 0-2: A and V in shared memory (<= 48 KiB, <= 100 KiB, <= ~226 KiB)
@@ -265,7 +267,8 @@ __device__ __noinline__ void tall_rounds(ColA colA, double *V, int m, int n, dou
 
 // What a kernel knows about its members' rows: nothing, at most kLanes, at
 // most kLanes / 2, or that they vary (the loops for every bound in one kernel,
-// which costs the longest of them their registers).
+// which costs the longest of them their registers).  At 512 threads one kernel
+// spills: any rows, A and V in global memory (72 bytes stored, 56 loaded).
 enum BatchRows { kRowsAny, kRows256, kRows128, kRowsVary };
 
 __host__ __device__ constexpr BatchRows batch_rows(int m)
@@ -495,7 +498,9 @@ __global__ void __launch_bounds__(256) batch_finish_kernel(const StepDesc *__res
 // two where their shape allows it (cluster_choice).  Registers decide
 // the rest: at two CTAs per SM a thread has 80, and with the member's shape and
 // the ring indices of every buffer kept in them the loops' own values went to
-// local memory (5.2 us per round; in shared memory now, ClusterRound).  100
+// local memory (5.2 us per round; in shared memory now, ClusterRound; 12 to 16
+// bytes still spill, 64 stored and 96 loaded in the form for more than 256 rows,
+// which cluster_choice takes the less often).  100
 // members: 21.5 ms, 31.3 on one CTA each; an SM per CTA with two slots in half
 // of its warps took 29.
 

@@ -724,6 +724,9 @@ __device__ __forceinline__ void evd_w_round(EvdRow &w, const double2 *cs, int q,
 // queues).  The G warps': shared-memory traffic, 48
 // KB per round, with each thread's loads issued before its stores.  Per round
 // (B200) 1670 cycles before, 950 now; per launch of 16 pairs 67 us, 39-40 now.
+// 24 warps leave a thread 80 registers, and the kernel spills (158 bytes stored,
+// 164 loaded, in the round loop too: 18 of a round's 1060 warp instructions go to
+// local memory).  20 warps would allow 96 registers and leave 15 for the bulk.
 // Writes W (64 x 64, column-major) - and, when Wimg is not null, its 3xTF32
 // operand image for the tensor-core rotation - and flags[pair] = 1 when some
 // pair rotated (else flags[pair] = 0 and W is left as it was).  stats[0] (as
