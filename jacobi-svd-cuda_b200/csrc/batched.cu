@@ -33,7 +33,9 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 #include "batch_tuning_table.h"
@@ -927,6 +929,9 @@ struct ClusterChoice {
     bool share = false;
 };
 
+// Work of one member per sweep, ~ n^2 (m + n): the queue order inside a class.
+double member_work(int m, int n) { return (double)n * n * (m + n); }
+
 // Clusters that the device holds at once: own[i] of 2 << i CTAs with an SM each,
 // shared4 of four CTAs at two to an SM.
 struct ClusterCapacity {
@@ -948,10 +953,10 @@ struct ClusterCapacity {
 // that eight shared CTAs where they keep the warps busy (9 to 12 slots on 12
 // warps).  More members: in class 4 two CTAs where they hold the member, four
 // shared ones where those keep the warps busy, else eight shared ones or the
-// smallest that holds it.  In class 3 whichever takes less, by whole waves: a wave
-// of the class's kernel lasts 1.5 to 1.6 waves of two CTAs (more than 256 rows:
-// 1.7 to 2.2), 2.4 of four.
-ClusterChoice cluster_choice(int m, int n, int cls, long members, size_t smem_cap, const ClusterCapacity &cap)
+// smallest that holds it.  In class 3 the smallest, or the class's kernel, as
+// clusters_sooner decides for the class.
+ClusterChoice cluster_choice(int m, int n, int cls, long members, bool sooner, size_t smem_cap,
+                             const ClusterCapacity &cap)
 {
     const int half = (n + (n & 1)) / 2;
     auto own = [&](int C) {  // at least two slots per CTA
@@ -962,15 +967,11 @@ ClusterChoice cluster_choice(int m, int n, int cls, long members, size_t smem_ca
         return half >= 2 * C && slots >= least && slots <= kClusterThreadsShared / 32 &&
                cluster_smem_bytes(m, n, C) <= smem_cap / 2 - 1024;
     };
-    auto waves = [&](int at_once) { return (members + at_once - 1) / std::max(at_once, 1); };
     if (own(8) && members <= cap.own[2]) return {8, false};
     if (shared(8, 9) && 8 * members <= 2 * cap.sms) return {8, true};
     if (own(4) && members <= cap.own[1]) return {4, false};
     const int C = own(2) ? 2 : (own(4) ? 4 : (own(8) ? 8 : 0));
-    if (cls == 3) {
-        const int tenths = C == 2 ? (m > kLanes ? 17 : 15) : (C == 4 ? 24 : 40);
-        return C > 0 && 10 * waves(cap.own[C / 4]) <= tenths * waves(cap.sms) ? ClusterChoice{C, false} : ClusterChoice{};
-    }
+    if (cls == 3) return sooner ? ClusterChoice{C, false} : ClusterChoice{};
     if (C == 2) {
         if (shared(4, 9) && (members <= cap.shared4 || members > cap.own[0])) return {4, true};
         return {2, false};
@@ -978,6 +979,50 @@ ClusterChoice cluster_choice(int m, int n, int cls, long members, size_t smem_ca
     // (8 slots: 512 x 128 7.3 ms against 8.0 for 37 members, 76 against 72 for 592)
     if (shared(8, 2 * members <= cap.sms ? 8 : 9)) return {8, true};
     return {C, false};
+}
+
+// Last end of jobs of the given lengths on `at_once` workers, each job taken by
+// the first free one, as the work queue does.
+double makespan(const std::vector<double> &lengths, int at_once)
+{
+    std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
+    double last = 0.0;
+    for (double t : lengths) {
+        if ((int)ends.size() == std::max(at_once, 1)) {
+            t += ends.top();
+            ends.pop();
+        }
+        ends.push(t);
+        last = std::max(last, t);
+    }
+    return last;
+}
+
+// Whether the smallest clusters that hold them solve the members of class 3 (in
+// queue order, by work) sooner than the class's kernel does.  A member takes 1.5
+// to 1.6 times as long on that kernel as on two CTAs, 1.7 to 2.2 times with more
+// than 256 rows, 2.4 times as long as on four (B200); the device holds twice or
+// four times as many of them.  So few members, and equal ones that fill the
+// kernel's last wave badly, go to clusters (300 of 270 x 100: 18.2 ms, 23.9 on
+// the class's kernel), ragged ones in number do not (211 of 100 to 226 KiB: 25.3
+// ms, 45).
+bool clusters_sooner(const std::vector<int> &members, const std::vector<BatchDesc> &all, size_t smem_cap,
+                     const ClusterCapacity &cap)
+{
+    if (members.size() > 8 * (size_t)cap.sms) return false;
+    std::vector<double> single, cluster[3];
+    for (int i : members) {
+        const int m = all[i].m, n = all[i].n;
+        const double t = member_work(m, n);
+        single.push_back(t);
+        int c = 0;
+        while (c < 3 && cluster_smem_bytes(m, n, 2 << c) > smem_cap) ++c;
+        if (c == 3) return false;
+        cluster[c].push_back(t / (c == 0 ? (m > kLanes ? 1.8 : 1.5) : (c == 1 ? 2.4 : 4.0)));
+    }
+    double ends = 0.0;
+    for (int c = 0; c < 3; ++c) ends += makespan(cluster[c], cap.own[c]);
+    return ends < 0.97 * makespan(single, cap.sms);
 }
 
 int cluster_capacity(int dev, int sms, size_t smem_cap, ClusterCapacity &cap)
@@ -1086,9 +1131,6 @@ int member_class(int m, int n, size_t smem_cap, size_t *smem_need)
         *smem_need = scratch + (class_a_shared(c) ? a_bytes : 0) + (class_v_shared(c) ? v_bytes : 0);
     return c;
 }
-
-// Work of one member per sweep, ~ n^2 (m + n): the queue order inside a class.
-double member_work(int m, int n) { return (double)n * n * (m + n); }
 
 // Argument checks shared by the solver and the autotuner.
 int check_batch_args(int count, const int *rows, const int *cols, const long long *a_offsets, const void *d_a,
@@ -1204,9 +1246,10 @@ int batch_solve(const BatchRequest &req, cudaStream_t stream)
         std::vector<int> sub[15];
         // (a launch shape given for class 3 is its own kernel's)
         const bool on = (mask >> c) & 1 && !(c == 3 && req.tuning != nullptr && req.tuning[3].threads > 0);
+        const bool sooner = on && c == 3 && clusters_sooner(members[c], all, smem_cap, capacity);
         for (int i : members[c]) {
             ClusterChoice cc;
-            if (on) cc = cluster_choice(all[i].m, all[i].n, c, (long)members[c].size(), smem_cap, capacity);
+            if (on) cc = cluster_choice(all[i].m, all[i].n, c, (long)members[c].size(), sooner, smem_cap, capacity);
             const BatchRows rows = c <= 2 ? batch_rows(all[i].m) : std::min(batch_rows(all[i].m), kRows256);
             sub[cc.C == 0 ? (int)rows
                           : (cc.C == 2 ? 3 : (cc.C == 4 ? 4 : 5)) + (cc.share ? 3 : 0) + (all[i].m > kLanes ? 6 : 0)]

@@ -87,3 +87,26 @@ def test_bytes_of_overlapping_groups(cuda_device, copies):
             w = want[i % len(want)]
             assert sw == w.sweeps
             assert np.array_equal(s, w.sigma) and np.array_equal(u, w.u) and np.array_equal(v, w.v)
+
+
+@pytest.mark.parametrize("count", [45, 100, 211])
+def test_many_ragged_members_of_class_3_keep_its_kernel_where_it_is_faster(cuda_device, count):
+    """Ragged members of class 3: with clusters allowed for the class
+    at most as long as without (a tenth for the spread of the runs).  A rule by
+    whole waves of equal members took 1.8 times as long for 211."""
+    rng = np.random.default_rng(count)
+    mats = []
+    while len(mats) < count:
+        m = int(rng.integers(100, 257))
+        n = int(rng.integers(8, m + 1))
+        if 8 * m * n < 222 * 1024 and 8 * (m * n + n * n) > 227 * 1024:
+            mats.append(rng.standard_normal((m, n)))
+    cfg = jsvd.default_config(epsilon=1e-12)
+    b = jsvd.DeviceBatch(mats, cuda_device)
+    chosen = _best_ms(b, cfg, reps=3)
+    old = jsvd.batch_set_cluster_classes(1 << 4)
+    try:
+        kernel = _best_ms(b, cfg, reps=3)
+    finally:
+        jsvd.batch_set_cluster_classes(old)
+    assert chosen <= 1.1 * kernel
